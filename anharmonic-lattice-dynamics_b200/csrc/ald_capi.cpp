@@ -427,6 +427,49 @@ static int v3_soft_fp64(ald_ctx* c, const V3Args& a, int* nl) {
   return ALD_OK;
 }
 
+// device bytes of one chunk of IBZ rows
+static size_t chunk_budget(const ald_ctx* c) { return c->opt.chunk_bytes ? c->opt.chunk_bytes : (size_t)512 << 20; }
+
+static V3LineTables v3_line_tables(const ald_ctx* c) {
+  V3LineTables t;
+  t.ns2 = c->VL.ns2;
+  t.ns3 = c->VL.ns3;
+  t.cls = c->ln_cls.p;
+  t.s2_off = c->ln_s2_off.p;
+  t.s3_off = c->ln_s3_off.p;
+  t.grp_off = c->ln_grp_off.p;
+  t.ph0 = c->ln_ph0.p;
+  t.ph1 = c->ln_ph1.p;
+  t.ph2 = c->ln_ph2.p;
+  return t;
+}
+
+// the row workspace and the line sums of nrows rows
+static int v3_line_alloc(ald_ctx* c, int nrows) {
+  const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, nrows, ALD_FP64);
+  if (c->w_h.n < need) CKA(c->w_h.alloc(need));
+  const size_t wb = v3_line_work_bytes(c->geo, v3_line_tables(c), nrows, c->opt.precision);
+  if (c->w_v3work.n < wb) CKA(c->w_v3work.alloc(wb));
+  return ALD_OK;
+}
+
+int v3_gauss_rows(ald_ctx* c) {
+  if (!v3_line_supported(c->geo, v3_line_tables(c), c->opt.precision)) return 0;
+  const size_t per_row = v3_hbuf_bytes(c->geo.b, c->VC.ncls, 1, ALD_FP64) +
+                         v3_line_row_bytes(c->geo, v3_line_tables(c), c->opt.precision);
+  return (int)std::max<size_t>(1, std::min<size_t>(chunk_budget(c) / per_row, (size_t)c->T.nibz));
+}
+
+int run_v3_gauss(ald_ctx* c, const V3Args& a0, const CombineArgs& ca, int* nlaunch) {
+  const int r = v3_line_alloc(c, a0.nrows);
+  if (r) return r;
+  V3Args a = a0;
+  a.hbuf = c->w_h.p;
+  CK(launch_v3_line_gauss(a, v3_line_tables(c), c->w_v3work.p, c->opt.precision, ca, c->stream));
+  *nlaunch += 4;
+  return ALD_OK;
+}
+
 int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
   int nl = 0;
   if (c->S.include_fc[2] != 1) return fail(ALD_ERR_ARG, "fc3 terms are not included (include_fc(3) /= 1)");
@@ -471,22 +514,13 @@ int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
     if (e == cudaSuccess) e = launch_v3_dense(a, c->w_v3work.p, c->w_v3work.n, c->stream);
     const long long per = (long long)(c->w_v3work.n / (2 * (size_t)c->geo.b * c->geo.b * c->geo.b * 16));
     nl += 1 + 3 * (int)(((long long)a.nrows * c->geo.nkc + per - 1) / per);
-  } else if (prec == ALD_MIXED && v3_tc_supported(c->geo.b, c->VC.ncls)) {
-    const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, a.nrows, prec);
-    if (c->w_h.n < need) CKA(c->w_h.alloc(need));
+  } else if (v3_line_supported(c->geo, v3_line_tables(c), prec)) {
+    // 3 bands: class sums axis by axis
+    const int r = v3_line_alloc(c, a.nrows);
+    if (r) return r;
     a.hbuf = c->w_h.p;
-    if (!c->ptiles_ok) {
-      CKA(c->w_ptiles.alloc(v3_tc_ptile_bytes(c->geo.nkc, c->VC.ncls)));
-      e = launch_v3_tc_ptiles(a, c->w_ptiles.p, c->stream);
-      if (e != cudaSuccess) return fail(ALD_ERR_CUDA, std::string("V3 phase tiles: ") + cudaGetErrorString(e));
-      c->ptiles_ok = true;
-      nl += 1;
-    }
-    const size_t bneed = v3_tc_btile_bytes(a.nrows, c->VC.ncls, c->geo.nkc);
-    if (c->w_btiles.n < bneed) CKA(c->w_btiles.alloc(bneed));
-    e = launch_v3_rows_f32(a, c->stream);
-    if (e == cudaSuccess) e = launch_v3_tc(a, c->w_ptiles.p, c->w_btiles.p, c->stream, c->tune_v3_rpc, c->tune_v3_wg);
-    nl += 4;  // class sums H, mode factors, B tiles, the MMA kernel
+    e = launch_v3_line(a, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
+    nl += 4;  // mode factors, class sums H, plane sums, the line kernel
   } else if (v3_pair_supported(c->geo.b, prec)) {
     const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, a.nrows, prec);
     if (c->w_h.n < need) CKA(c->w_h.alloc(need));
@@ -552,8 +586,7 @@ double gauss_width(ald_ctx* c) { return c->opt.width_cm > 0 ? c->opt.width_cm : 
 // |V3|^2 rows per chunk within the byte budget
 int rows_per_chunk(ald_ctx* c) {
   size_t per_row = (size_t)c->T.nkc * c->geo.b * c->geo.b * c->geo.b * sizeof(double);
-  size_t budget = c->opt.chunk_bytes ? c->opt.chunk_bytes : (size_t)512 << 20;
-  return (int)std::max<size_t>(1, std::min<size_t>(budget / per_row, (size_t)c->T.nibz));
+  return (int)std::max<size_t>(1, std::min<size_t>(chunk_budget(c) / per_row, (size_t)c->T.nibz));
 }
 
 }  // namespace capi
@@ -684,6 +717,17 @@ int ald_create_from_dir(const char* dir, const ald_options* opt, ald_ctx** out) 
       }
     }
     st.add(c->roots, rt);
+    if (c->S.include_fc[2] == 1 && c->T.b == 3) {
+      V3Lines& ln = c->VL;
+      build_v3_lines(c->S, c->T, c->VC, rt, ln);
+      st.add(c->ln_cls, ln.cls);
+      st.add(c->ln_s2_off, ln.s2_off);
+      st.add(c->ln_s3_off, ln.s3_off);
+      st.add(c->ln_grp_off, ln.grp_off);
+      st.add(c->ln_ph0, ln.ph0);
+      st.add(c->ln_ph1, ln.ph1);
+      st.add(c->ln_ph2, ln.ph2);
+    }
   }
   st.add(c->phase_coef, c->T.phase_coef);
   std::vector<int> mi(c->T.nibz);

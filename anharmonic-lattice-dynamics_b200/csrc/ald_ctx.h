@@ -12,6 +12,7 @@ struct ald_ctx {
   Tables T;
   Fc3Blocks F3;
   V3Classes VC;
+  V3Lines VL;  // its counts and offsets (the phase tables stay on the device)
   Fc2Csr F2;
   ald_options opt;
   int device = 0;
@@ -26,19 +27,18 @@ struct ald_ctx {
   DevBuf<int> fc2_off, fc2_atom, blk_off, trip_j, trip_k, phase_coef, mapinv, neg_src, neg_dst, arm_off, arm_q,
       arm_op, star_off, star_q, star_op, tet_corner, tet_inc, err;
   DevBuf<int> cls_grp_off, cls_pc, cls_trip_off, cls_trip, cls_trip_i0, cls_trip_k;
+  DevBuf<int> ln_cls, ln_s2_off, ln_s3_off, ln_grp_off;
+  DevBuf<double> ln_ph0, ln_ph1, ln_ph2;
   DevBuf<int> arm_owner;              // per arm: its IBZ point (kappa over arms)
   DevBuf<int> mesh_m;                 // per mesh point: its three mesh integers (+ 1 pad)
   DevBuf<int> mapibz0, full_op;       // per mesh point: IBZ point and the op of its star arm (job=3)
   bool full_op_ok = false;
   DevBuf<char> w_h;                   // per-row phase-class sums of the pair kernel
-  DevBuf<char> w_ptiles;              // phase tiles of the tensor-core V3 (mesh-only, built once)
-  DevBuf<char> w_btiles;              // per-row B operands of the tensor-core V3
-  DevBuf<char> w_v3work;              // T1/T2 of the large-cell V3 GEMMs
+  DevBuf<char> w_v3work;              // T1/T2 of the large-cell V3 GEMMs; line sums of the 3-band V3
   DevBuf<char> w_h64, w_v3fix;        // mixed path, FP64 V3 near zero frequencies: H and T1/T2
   DevBuf<long long> w_pairs;          // its (row, q2) pair list
   int v3work_tc_b = 0;                // its tensor-core T2 padding is zero for (bands, pairs)
   long long v3work_tc_p = 0;
-  bool ptiles_ok = false;
   // phonons and occupations
   DevBuf<double> w2_all, w2, evec, vel, freq, dist;
   // pipeline workspaces, kept across calls (allocation outside the timed work)
@@ -54,7 +54,7 @@ struct ald_ctx {
   DevBuf<double> w_heev;    // Householder eigensolver workspace (large cells)
   DevBuf<double> w_rmax;    // deterministic delta: each R entry's largest term (FP64 bits)
   // launch shapes chosen by ald_autotune (0 = the built-in choices)
-  int tune_v3_rpc = 0, tune_v3_wg = 0;
+  int tune_v3_rpc = 0, tune_v3_wg = 0;  // kept for ald_set_tuning's callers; nothing reads them
   size_t tune_gemm_bytes = 0;
   CgWork cg;
   bool have_phonons = false;
@@ -79,6 +79,10 @@ int ensure_dist(ald_ctx* c, double tempk);
 V3Args v3_args(ald_ctx* c, int first, int nrows, double* out);
 // nlaunch (optional) += the kernels launched
 int run_v3(ald_ctx* c, const V3Args& a, int* nlaunch);
+// V3 and the Gaussian delta in one pass: rows per chunk (their line sums within
+// the chunk's byte budget), 0 where the cell has no such kernel
+int v3_gauss_rows(ald_ctx* c);
+int run_v3_gauss(ald_ctx* c, const V3Args& a, const CombineArgs& ca, int* nlaunch);
 // g of cal_giso on the device (the element table unless ald_set_isotope_g set it)
 int ensure_giso(ald_ctx* c);
 KappaArgs kappa_args(ald_ctx* c, double tempk);

@@ -1049,6 +1049,52 @@ std::string build_v3_classes(const System& S, const Tables& T, const Fc3Blocks& 
   return "";
 }
 
+void build_v3_lines(const System& S, const Tables& T, const V3Classes& C, const std::vector<double>& roots,
+                    V3Lines& Lo) {
+  const int L = T.L, ngrp = (int)C.grp_off.size() - 1;
+  Lo = V3Lines();
+  Lo.cls.resize(C.ncls);
+  std::iota(Lo.cls.begin(), Lo.cls.end(), 0);
+  Lo.s2_off.assign(1, 0);
+  Lo.s3_off.assign(1, 0);
+  Lo.grp_off.assign(1, 0);
+  std::vector<int> c1, c2;  // axis-1 coefficient of each slot 2, axis-2 coefficient of each slot 3
+  for (int g = 0; g < ngrp; ++g) {
+    const int lo = C.grp_off[g], hi = C.grp_off[g + 1];
+    auto key = [&](int c) { return std::make_pair(C.pc[4 * (size_t)c + 2], C.pc[4 * (size_t)c + 1]); };
+    std::stable_sort(Lo.cls.begin() + lo, Lo.cls.begin() + hi, [&](int x, int y) { return key(x) < key(y); });
+    for (int n = lo; n < hi; ++n) {
+      const bool new3 = n == lo || key(Lo.cls[n]).first != key(Lo.cls[n - 1]).first;
+      if (n > lo && key(Lo.cls[n]) != key(Lo.cls[n - 1])) Lo.s2_off.push_back(n);
+      if (n > lo && new3) Lo.s3_off.push_back((int)Lo.s2_off.size() - 1);
+      if (new3) c2.push_back(key(Lo.cls[n]).first);
+      if (n == lo || key(Lo.cls[n]) != key(Lo.cls[n - 1])) c1.push_back(key(Lo.cls[n]).second);
+    }
+    if (hi > lo) {
+      Lo.s2_off.push_back(hi);
+      Lo.s3_off.push_back((int)Lo.s2_off.size() - 1);
+    }
+    Lo.grp_off.push_back((int)Lo.s3_off.size() - 1);
+  }
+  Lo.ns2 = (int)c1.size();
+  Lo.ns3 = (int)c2.size();
+  auto fill = [&](std::vector<double>& ph, int n, size_t count, auto index) {
+    ph.resize(2 * (size_t)n * count);
+    for (int m = 0; m < n; ++m)
+      for (size_t k = 0; k < count; ++k) {
+        const long long t = index((long long)m, k) % L;
+        ph[2 * (m * count + k)] = roots[2 * t];
+        ph[2 * (m * count + k) + 1] = roots[2 * t + 1];
+      }
+  };
+  fill(Lo.ph0, S.nc[0], Lo.cls.size(), [&](long long m, size_t k) {
+    const int* pc = &C.pc[4 * (size_t)Lo.cls[k]];
+    return m * pc[0] + pc[3];
+  });
+  fill(Lo.ph1, S.nc[1], c1.size(), [&](long long m, size_t k) { return m * c1[k]; });
+  fill(Lo.ph2, S.nc[2], c2.size(), [&](long long m, size_t k) { return m * c2[k]; });
+}
+
 std::string build_fc2(const System& S, Fc2Csr& F) {
   int b = 3 * S.nat0;
   int nt = (int)S.f2.size();

@@ -127,6 +127,22 @@ struct V3Classes {
 };
 std::string build_v3_classes(const System& S, const Tables& T, const Fc3Blocks& F, V3Classes& C);
 
+// The classes ordered for sums taken axis by axis (ald_v3_line.cu).  Within a
+// group, the classes that share the axis-2 phase are a "slot 3" and, of
+// those, the ones that also share the axis-1 phase a "slot 2".
+struct V3Lines {
+  int ns2 = 0, ns3 = 0;
+  std::vector<int> cls;       // class at each place of the order
+  std::vector<int> s2_off;    // ns2 + 1: places of each slot 2
+  std::vector<int> s3_off;    // ns3 + 1: slots 2 of each slot 3
+  std::vector<int> grp_off;   // nat0^2 + 1: slots 3 of each group
+  // phases (re, im) of the mesh integers: [m_0][place] with the class's shift
+  // term, [m_1][slot 2], [m_2][slot 3]
+  std::vector<double> ph0, ph1, ph2;
+};
+void build_v3_lines(const System& S, const Tables& T, const V3Classes& C, const std::vector<double>& roots,
+                    V3Lines& Lo);
+
 // FC2 grouped per dynamical-matrix element (i3, j3) in the file's term
 // order (the order set_dynamical_matrix sums them).
 struct Fc2Csr {
@@ -305,11 +321,28 @@ struct V3Args {
   long long npairs_list = 0;
 };
 cudaError_t launch_v3_fp64(const V3Args& a, cudaStream_t s);
+// 3 and 6 bands, class sums axis by axis (ald_v3_line.cu): V3Lines on the
+// device; hbuf of v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) bytes and work of
+// v3_line_work_bytes (per-mode factors, the row's sums per mesh line)
+struct V3LineTables {
+  int ns2, ns3;
+  const int* cls;
+  const int* s2_off;
+  const int* s3_off;
+  const int* grp_off;
+  const double* ph0;
+  const double* ph1;
+  const double* ph2;
+};
+bool v3_line_supported(const Geometry& g, const V3LineTables& t, int precision);
+size_t v3_line_row_bytes(const Geometry& g, const V3LineTables& t, int precision);
+size_t v3_line_work_bytes(const Geometry& g, const V3LineTables& t, int nrows, int precision);
+cudaError_t launch_v3_line(const V3Args& a, const V3LineTables& t, void* work, int precision, cudaStream_t s);
 // pair kernel: bands it handles and the row workspace it needs (0 = not handled)
 bool v3_pair_supported(int b, int precision);
 size_t v3_hbuf_bytes(int b, int ncls, int nrows, int precision);
 cudaError_t launch_v3_pair(const V3Args& a, int precision, cudaStream_t s);
-// row stage alone, H in FP32 (for the tensor-core class sums) or FP64
+// row stage alone, H in FP32 or FP64
 cudaError_t launch_v3_rows_f32(const V3Args& a, cudaStream_t s);
 cudaError_t launch_v3_rows_f64(const V3Args& a, cudaStream_t s);
 // more than 12 bands (ald_v3_dense.cu): the class sums and both mode products
@@ -334,19 +367,6 @@ cudaError_t launch_v3_dense_tc(const V3Args& a, void* work, long long pairs, boo
 // the |V3|^2 layout the pipeline asks V3 for and hands to the delta:
 // 0 [row][q2][l1][l2][l3], 1 [row][l2][l3][l1][q2], 2 [row][l2][l3][q2][l1]
 int v3_pipeline_layout(int b, int precision);
-// 3 bands, ALD_MIXED: class sums on tcgen05 (ald_v3_tc.cu); hbuf from launch_v3_rows_f32
-bool v3_tc_supported(int b, int ncls);
-// the row-independent phase tiles (split FP16, canonical layout), built once per context
-size_t v3_tc_ptile_bytes(int nkc, int ncls);
-cudaError_t launch_v3_tc_ptiles(const V3Args& a, void* ptiles, cudaStream_t s);
-// btiles: scratch of v3_tc_btile_bytes(nrows, ncls, nkc) (B operands and row data of the
-// chunk's rows, per-mode factors and FP32 eigenvectors of the mesh)
-size_t v3_tc_btile_bytes(int nrows, int ncls, int nkc);
-// rows_per_cta, epilogue_wg: 0 = the built-in choice (up to 16 rows while the
-// grid fills the GPU twice; 2 warpgroups), else 1..16 rows and 2 or 3
-cudaError_t launch_v3_tc(const V3Args& a, const void* ptiles, void* btiles, cudaStream_t s, int rows_per_cta = 0,
-                         int epilogue_wg = 0);
-
 struct CombineArgs {
   Geometry geo;
   int n1_first, nrows;
@@ -378,6 +398,11 @@ struct CombineArgs {
   double* P1;                // optional Bose-weighted
   double* P2;
 };
+// V3 and the Gaussian delta of a chunk in one pass (3 bands): R1, R2 of the
+// rows, |V3|^2 is not stored.  ca.f32w goes with the precision; no R1p/R2p,
+// P1s/P2s, P1/P2
+cudaError_t launch_v3_line_gauss(const V3Args& a, const V3LineTables& t, void* work, int precision,
+                                 const CombineArgs& ca, cudaStream_t s);
 // scratch: the corner energies of the chunk (combine_scratch_bytes)
 size_t combine_scratch_bytes(const Geometry& geo, int nrows, int gauss);
 cudaError_t launch_combine(const CombineArgs& a, void* scratch, cudaStream_t s);

@@ -205,9 +205,16 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   // V3 of 3 and 6 bands into the fused tetrahedron delta.  Half the bytes,
   // twice the rows per chunk.
   const bool v3f = v3_layout == 2 || (mixed && fused && v3_layout == 1 && (b == 3 || b == 6));
-  const int K = v3f ? std::min(nibz, 2 * rows_per_chunk(c)) : rows_per_chunk(c);
+  int K = v3f ? std::min(nibz, 2 * rows_per_chunk(c)) : rows_per_chunk(c);
   const size_t v3n = (size_t)K * nkc * b * b * b;
-  ALD_CKA(v3.alloc(v3f ? (v3n + 1) / 2 : v3n));
+  // where |V3|^2 takes several chunks it is not kept after the call, and a
+  // cell with a kernel for V3 and the Gaussian delta together never stores it
+  // (its chunks are cut by that kernel's own workspace).  argon 32^3 mixed, V3
+  // and delta: 19.4 ms in two kernels, 11.9 in one; 26^3 FP64: 14.8 and 8.5
+  const bool one_chunk = re - rb <= K;
+  const bool v3_gauss = gauss && !it && !one_chunk && v3_gauss_rows(c) > 0;
+  if (v3_gauss) K = v3_gauss_rows(c);
+  if (!v3_gauss) ALD_CKA(v3.alloc(v3f ? (v3n + 1) / 2 : v3n));
   const size_t rchunk = (size_t)K * nkc * b * b;  // entries of one chunk's R1
   if (det) ALD_CKA(c->w_rmax.alloc((it ? 4 : 2) * rchunk));
   if (!fused && !any) ALD_CKA(escratch.alloc(std::max<size_t>(256, combine_scratch_bytes(c->geo, K, gauss))));
@@ -216,7 +223,6 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   res->launches[0] += 1;  // band ranges of the occupations, outside the timed delta stage
   // one chunk holds every row: |V3|^2 kept from an earlier call with the same
   // eigenpairs and rows is reused (a run over several temperatures forms it once)
-  const bool one_chunk = re - rb <= K;
   const bool v3_kept = one_chunk && c->v3c_epoch != 0 && c->v3c_epoch == c->phonon_epoch && c->v3c_rb == rb &&
                        c->v3c_re == re && c->v3c_layout == v3_layout && c->v3c_f32 == v3f && c->v3c_ptr == v3.p &&
                        c->v3c_n == v3.n;
@@ -224,7 +230,7 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   for (int r0 = rb; r0 < re; r0 += K) {
     int nr = std::min(K, re - r0);
     ALD_CK(tm.begin(1));
-    if (!v3_kept) {
+    if (!v3_kept && !v3_gauss) {
       V3Args va = v3_args(c, r0, nr, v3.p);
       va.v3_layout = v3_layout;
       if (v3f) va.v3sq_f32 = reinterpret_cast<float*>(v3.p);
@@ -282,7 +288,10 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
       ALD_CK(cudaMemsetAsync(a.R2, 0, rbytes, s));
     }
     ALD_CK(tm.begin(2));
-    if (det) {
+    if (v3_gauss) {
+      r = run_v3_gauss(c, v3_args(c, r0, nr, nullptr), a, &res->launches[2]);
+      if (r) return r;
+    } else if (det) {
       const size_t n = (size_t)nr * nkc * b * b;
       ALD_CK(launch_delta_fused(a, s, 1));
       ALD_CK(launch_delta_fused(a, s, 2));
@@ -550,7 +559,6 @@ static void release_pipeline_workspaces(ald_ctx* c) {
   c->w_pairs.free();
   c->w_v3work.free();
   c->v3work_tc_b = 0;
-  c->w_btiles.free();
   c->w_scratch.free();
 }
 

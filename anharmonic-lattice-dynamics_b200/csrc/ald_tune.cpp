@@ -10,14 +10,13 @@
 // the current choice:
 //   1. the |V3|^2 chunk (IBZ rows per V3 and delta launch; 256 MiB .. 2 GiB,
 //      within a quarter of the free device memory);
-//   2. mixed path, 3 bands: the tensor-core V3's IBZ rows per CTA (phase-tile
-//      reuse against grid size) and its epilogue warpgroups (2 or 3);
-//   3. mixed path, 9 bands and up: the pair-batch workspace of the
+//   2. mixed path, 9 bands and up: the pair-batch workspace of the
 //      tensor-core mode-product GEMMs (launch count against L2 reuse).
 // The best choice stays on the context and goes into the cache file as one
 // line "<shape> chunk_bytes=.. rpc=.. wg=.. gemm_bytes=.. ms=..", replaced
 // in place when the shape is tuned again; a later call for the same shape
-// reads it instead of timing.  Every knob changes launch shapes only: the
+// reads it instead of timing.  (rpc and wg, knobs of an earlier 3-band V3,
+// are carried through and have no effect.)  Every knob changes launch shapes only: the
 // per-pair and per-row arithmetic, and so the results, stay the same.
 #include <cuda_runtime.h>
 
@@ -220,18 +219,7 @@ int ald_autotune(ald_ctx* c, const char* cache_path, double budget_s, ald_tuning
     r = trial(ch);
     if (r) break;
   }
-  // 2. 3-band tensor-core V3: rows per CTA x epilogue warpgroups
-  if (!r && c->opt.precision == ALD_MIXED && v3_tc_supported(c->geo.b, c->VC.ncls)) {
-    const Choice base = best;
-    for (int rpc : {2, 4, 8, 16})
-      for (int wg : {2, 3}) {
-        Choice ch = base;
-        ch.rpc = rpc;
-        ch.wg = wg;
-        if (!r) r = trial(ch);
-      }
-  }
-  // 3. large cells: the GEMM pair-batch workspace
+  // 2. large cells: the GEMM pair-batch workspace
   if (!r && c->opt.precision == ALD_MIXED && v3_dense_tc_supported(c->geo.b)) {
     const Choice base = best;
     for (size_t mb : {512, 1024, 4096}) {

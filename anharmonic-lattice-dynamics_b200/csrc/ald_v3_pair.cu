@@ -100,6 +100,9 @@ __global__ void v3_row_kernel(V3Args a) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
     const int l1 = e % b, bg = (e / b) % 9, c = e / (9 * b);
     double2 acc = make_double2(0.0, 0.0);
+    // unrolled so that the loads of several members overlap (the class of
+    // R_j = R_k has one member per neighbour)
+#pragma unroll 4
     for (int s = a.cls_trip_off[c]; s < a.cls_trip_off[c + 1]; ++s) {
       const int t = a.cls_trip[s], i0 = a.cls_trip_i0[s], k = a.cls_trip_k[s];
       int ph = phase_index(a.phase_coef + 4 * k, m1, g.L, g.L32);

@@ -30,7 +30,7 @@ SOURCES = {
     "ald_heev.cu": [],
     "ald_v3.cu": [],
     "ald_v3_pair.cu": [],
-    "ald_v3_tc.cu": [],
+    "ald_v3_line.cu": [],
     "ald_v3_dense.cu": [],
     "ald_v3_dense_tc.cu": [],
     # weight_tet's FP32/FP64 arithmetic must not be contracted into FMAs

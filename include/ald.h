@@ -41,13 +41,13 @@ enum ald_status {
 
 enum ald_delta { ALD_DELTA_TETRA = 0, ALD_DELTA_GAUSS = 1 };
 /* ALD_MIXED: the V3 contraction in reduced precision with FP32 accumulation --
- * for 3 bands the phase-class sums, from 9 bands up both eigenvector mode
- * products run on the tensor cores (split-FP16 tcgen05 MMAs), 6 bands in FP32
- * on the CUDA cores; from 9 bands up the pairs that involve a mode of
- * vanishing frequency are formed again in FP64.  ALD_MIXED_FP32 uses the FP32
- * CUDA-core form where one exists.  Inside the pipeline the delta weights and
- * the stored collision matrix are FP32 too; eigensolve, Bose factors, the sums
- * into Q, CG vectors and kappa stay FP64. */
+ * from 9 bands up both eigenvector mode products run on the tensor cores
+ * (split-FP16 tcgen05 MMAs), 3 and 6 bands in FP32 on the CUDA cores; from 9
+ * bands up the pairs that involve a mode of vanishing frequency are formed
+ * again in FP64.  ALD_MIXED_FP32 uses the FP32 CUDA-core form where one
+ * exists.  Inside the pipeline the delta weights and the stored collision
+ * matrix are FP32 too; eigensolve, Bose factors, the sums into Q, CG vectors
+ * and kappa stay FP64. */
 enum ald_precision { ALD_FP64 = 0, ALD_MIXED = 1, ALD_MIXED_FP32 = 2 };
 enum ald_cg_stop { ALD_CG_REFERENCE = 0, ALD_CG_RESIDUAL = 1 };
 
@@ -257,7 +257,8 @@ typedef struct ald_kappa_result {
   int status_cg;           /* ALD_OK or ALD_WARN_CG_MAXITER              */
   double cg_err;           /* last error measure of the stop rule        */
   /* device time per stage (CUDA events on the context's stream), ms:
-     0 phonons+occupations, 1 V3, 2 delta+Bose+band sums, 3 Q reduce,
+     0 phonons+occupations, 1 V3, 2 delta+Bose+band sums (with V3 where one
+     kernel does both: 3 bands, Gaussian delta, several chunks), 3 Q reduce,
      4 RTA kappa, 5 collision matrix, 6 RHS, 7 CG, 8 CG kappa, 9 total   */
   double stage_ms[10];
   int launches[10];        /* kernel launches per stage (same indices)   */
@@ -304,8 +305,7 @@ int ald_kappa_batched(int n, ald_ctx* const* ctx, const double* tempk, ald_kappa
  * pipeline's autotuner.  ald_autotune times whole ald_kappa_pipeline calls
  * (device time, at the tmin of latdyn.params) over candidate launch shapes,
  * one knob at a time: the |V3|^2 chunk (IBZ rows per V3 and delta launch),
- * for 3-band mixed cells the tensor-core V3's rows per CTA and epilogue
- * warpgroups, for mixed cells of 9 bands and up the pair-batch workspace of
+ * and for mixed cells of 9 bands and up the pair-batch workspace of
  * the tensor-core mode-product GEMMs.  It keeps the fastest on the context
  * and in the cache file (cache_path; NULL or "": $ALD_TUNE_CACHE; neither:
  * no file), one text line per shape (device, bands, mesh, IBZ rows,
@@ -316,8 +316,8 @@ int ald_kappa_batched(int n, ald_ctx* const* ctx, const double* tempk, ald_kappa
  * the built-in choices). */
 typedef struct ald_tuning {
   size_t chunk_bytes;   /* as ald_options.chunk_bytes (0 = automatic)                    */
-  int v3_rows_per_cta;  /* 3-band tensor-core V3: IBZ rows per CTA, 1..16 (0 = built-in) */
-  int v3_epilogue_wg;   /* 3-band tensor-core V3: epilogue warpgroups, 2 or 3 (0 = 2)    */
+  int v3_rows_per_cta;  /* 0..16, carried through; no effect (an earlier 3-band V3)      */
+  int v3_epilogue_wg;   /* 0, 2 or 3, carried through; no effect                         */
   size_t v3_gemm_bytes; /* tensor-core mode-product GEMMs: pair-batch workspace (0 = 2 GiB) */
   double ms;            /* device time of one pipeline call with this choice             */
   int from_cache;       /* 1: read from the cache file, 0: timed by this call            */
