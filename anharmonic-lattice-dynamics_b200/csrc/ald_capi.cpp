@@ -265,8 +265,9 @@ int ensure_dist(ald_ctx* c, double tempk) {
   const size_t n = (size_t)c->geo.nkc * c->geo.b;
   CKA(c->freq.alloc(n));
   CKA(c->dist.alloc(n));
+  CKA(c->occt.alloc(2 * n));
   CK(launch_freq_dist(c->geo, c->w2.p, PhysConst::cnst(), temp_cm(tempk), c->S.classical, c->freq.p, c->dist.p,
-                      c->err.p, c->stream));
+                      c->occt.p, c->err.p, c->stream));
   int r = check_err_flags(c);
   if (r) return r;
   c->dist_tempk = tempk;
@@ -345,6 +346,8 @@ static int v3_soft_fp64(ald_ctx* c, const V3Args& a, int* nl) {
     m[1] = (q / nc[2]) % nc[1];
     m[2] = q % nc[2];
   };
+  // the kernel the FP64 path uses for this cell
+  const bool tile64 = v3_tile_supported(c->geo, c->VC.ncls, ALD_FP64);
   std::vector<long long> all, part;
   std::vector<int> soft_rows;  // rows of a soft q1 formed by the direct FP64 kernel
   int nk1 = 0;
@@ -367,7 +370,7 @@ static int v3_soft_fp64(ald_ctx* c, const V3Args& a, int* nl) {
     }
     if (nsoft[q1]) {
       nk1 = std::max(nk1, nsoft[q1]);
-      if (v3_dense_supported(b))
+      if (!tile64 && v3_dense_supported(b))
         for (int q2 = 0; q2 < nkc; ++q2) part.push_back((long long)r * nkc + q2);
       else
         soft_rows.push_back(r);
@@ -417,7 +420,14 @@ static int v3_soft_fp64(ald_ctx* c, const V3Args& a, int* nl) {
       g.v3sq = reinterpret_cast<double*>(c->w_v3fix.p);
       g.v3sq_f32 = nullptr;
       g.pair_list = nullptr;
-      e = launch_v3_fp64(g, c->stream);
+      if (tile64) {
+        const size_t wb = v3_tile_work_bytes(c->geo, c->VC.ncls, 1, ALD_FP64);
+        if (c->w_h64.n < wb) CKA(c->w_h64.alloc(wb));
+        e = launch_v3_tile(g, c->w_h64.p, ALD_FP64, c->stream, nk1);
+        *nl += 2;
+      } else {
+        e = launch_v3_fp64(g, c->stream);
+      }
       if (e == cudaSuccess) e = launch_v3_copy_row(a, r, g.v3sq, nk1, c->stream);
       *nl += 2;
       if (e != cudaSuccess) break;
@@ -443,6 +453,9 @@ static V3LineTables v3_line_tables(const ald_ctx* c) {
   t.ph2 = c->ln_ph2.p;
   return t;
 }
+
+bool v3_tile_used(const ald_ctx* c) { return v3_tile_supported(c->geo, c->VC.ncls, c->opt.precision); }
+int v3_layout(const ald_ctx* c) { return v3_tile_used(c) ? 1 : v3_pipeline_layout(c->geo.b, c->opt.precision); }
 
 // the row workspace and the line sums of nrows rows
 static int v3_line_alloc(ald_ctx* c, int nrows) {
@@ -478,7 +491,18 @@ int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
   const int prec = c->opt.precision;
   V3Args a = a0;
   cudaError_t e;
-  if (prec == ALD_MIXED && v3_dense_tc_supported(c->geo.b)) {
+  if (v3_tile_used(c) && a.v3_layout <= 1) {
+    // 9 bands and up, pairs in shared memory
+    const size_t wb = v3_tile_work_bytes(c->geo, c->VC.ncls, a.nrows, prec);
+    if (c->w_v3work.n < wb) CKA(c->w_v3work.alloc(wb));
+    c->v3work_tc_b = 0;
+    e = launch_v3_tile(a, c->w_v3work.p, prec, c->stream);
+    nl += 3;  // mode factors, class sums H, the pairs
+    if (e == cudaSuccess && prec == ALD_MIXED) {
+      const int r = v3_soft_fp64(c, a, &nl);
+      if (r) return r;
+    }
+  } else if (prec == ALD_MIXED && v3_dense_tc_supported(c->geo.b)) {
     // more than 12 bands, mixed: split-FP16 tensor-core GEMMs per pair
     const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, a.nrows, ALD_MIXED);
     if (c->w_h.n < need) CKA(c->w_h.alloc(need));

@@ -40,7 +40,7 @@ struct ald_ctx {
   int v3work_tc_b = 0;                // its tensor-core T2 padding is zero for (bands, pairs)
   long long v3work_tc_p = 0;
   // phonons and occupations
-  DevBuf<double> w2_all, w2, evec, vel, freq, dist;
+  DevBuf<double> w2_all, w2, evec, vel, freq, dist, occt;
   // pipeline workspaces, kept across calls (allocation outside the timed work)
   DevBuf<double> w_R1, w_R2, w_Q, w_v3, w_F, w_x, w_rhs, w_kr, w_kc, w_cm;
   DevBuf<double> w_R1p, w_R2p, w_Ff, w_Frta, w_part;  // iterative solution: band marginals, F on the mesh
@@ -79,6 +79,9 @@ int ensure_dist(ald_ctx* c, double tempk);
 V3Args v3_args(ald_ctx* c, int first, int nrows, double* out);
 // nlaunch (optional) += the kernels launched
 int run_v3(ald_ctx* c, const V3Args& a, int* nlaunch);
+// whether ald_v3_tile.cu forms this context's |V3|^2, and the layout the pipeline asks V3 for
+bool v3_tile_used(const ald_ctx* c);
+int v3_layout(const ald_ctx* c);
 // V3 and the Gaussian delta in one pass: rows per chunk (their line sums within
 // the chunk's byte budget), 0 where the cell has no such kernel
 int v3_gauss_rows(ald_ctx* c);

@@ -251,8 +251,9 @@ cudaError_t launch_phonon_post(const Geometry& geo, const double* w2_all, double
                                cudaStream_t s);
 cudaError_t launch_subst_eivecs(const Geometry& geo, const int* src, const int* dst, int n, double* evec,
                                 cudaStream_t s);
+// freq, dist [q][l]; occt: the same as [l][q], freq then dist
 cudaError_t launch_freq_dist(const Geometry& geo, const double* w2, double cnst, double temp, int classical,
-                             double* freq, double* dist, int* err, cudaStream_t s);
+                             double* freq, double* dist, double* occt, int* err, cudaStream_t s);
 
 // Three-phonon self-energy at arbitrary q (function_self_w3/w4), ald_self.cu
 struct SelfArgs {
@@ -364,9 +365,16 @@ long long v3_dense_tc_pairs(int b, long long npairs, size_t budget);
 size_t v3_dense_tc_work_bytes(int b, int nkc, int nrows, long long pairs);
 int v3_dense_tc_launches(long long npairs, long long pairs);
 cudaError_t launch_v3_dense_tc(const V3Args& a, void* work, long long pairs, bool a2_zeroed, cudaStream_t s);
-// the |V3|^2 layout the pipeline asks V3 for and hands to the delta:
+// the |V3|^2 layout the pipeline asks V3 for and hands to the delta, where
+// ald_v3_tile.cu does not take the cell:
 // 0 [row][q2][l1][l2][l3], 1 [row][l2][l3][l1][q2], 2 [row][l2][l3][q2][l1]
 int v3_pipeline_layout(int b, int precision);
+// 9 bands and up whose pairs fit shared memory (ald_v3_tile.cu), FP64 and
+// mixed; work of v3_tile_work_bytes; layouts 0 and 1.  l1_keep (0 = all): only
+// bands l1 < l1_keep
+bool v3_tile_supported(const Geometry& g, int ncls, int precision);
+size_t v3_tile_work_bytes(const Geometry& g, int ncls, int nrows, int precision);
+cudaError_t launch_v3_tile(const V3Args& a, void* work, int precision, cudaStream_t s, int l1_keep = 0);
 struct CombineArgs {
   Geometry geo;
   int n1_first, nrows;
@@ -376,6 +384,7 @@ struct CombineArgs {
   const float* v3sq_f32 = nullptr;  // FP32 |V3|^2 in place of v3sq (band-generic kernels only)
   const double* freq;        // [q][l]
   const double* dist;        // [q][l]
+  const double* occt = nullptr;  // freq, then dist, as [l][q] (delta_gauss_pair)
   const int* tet_corner;
   const int* tet_inc;
   int gauss;
@@ -422,6 +431,9 @@ cudaError_t launch_delta_finalize(double* R, const unsigned long long* M, size_t
 // R1/R2/P1s/P2s (and R1p/R2p) must be zero on entry; P1/P2 are not produced
 constexpr int kDeltaSmallBands = 16;  // up to here the band-templated kernels
 cudaError_t launch_delta_any(const CombineArgs& a, cudaStream_t s);
+// the Gaussian delta into R1/R2 alone, |V3|^2 in layout 1, 6 bands and up
+bool delta_gauss_pair_supported(const CombineArgs& a);
+cudaError_t launch_delta_gauss_pair(const CombineArgs& a, cudaStream_t s);
 // Q/QN/QU[(n1_first+row)*b + l1] from R1/R2 of rows [0, nrows)
 cudaError_t launch_q_from_r(const Geometry& geo, int n1_first, int nrows, const int* mapinv, const double* R1,
                             const double* R2, double* Q, double* QN, double* QU, int nibz, cudaStream_t s);

@@ -619,12 +619,18 @@ __device__ __forceinline__ double nbe_dev(double w, double t, int m, int* err) {
 }
 
 __global__ void freq_dist_kernel(Geometry geo, const double* w2, double cnst, double temp, int classical,
-                                 double* freq, double* dist, int* err) {
+                                 double* freq, double* dist, double* occt, int* err) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= geo.nkc * geo.b) return;
+  const int n = geo.nkc * geo.b;
+  if (idx >= n) return;
   double f = sqrt(w2[idx]) * cnst;
+  const double d = nbe_dev(f, temp, classical, err);
   freq[idx] = f;
-  dist[idx] = nbe_dev(f, temp, classical, err);
+  dist[idx] = d;
+  // the same band by band, for threads that walk q
+  const int q = idx / geo.b, t = (idx - q * geo.b) * geo.nkc + q;
+  occt[t] = f;
+  occt[n + t] = d;
 }
 
 }  // namespace
@@ -679,9 +685,9 @@ cudaError_t launch_subst_eivecs(const Geometry& geo, const int* src, const int* 
 }
 
 cudaError_t launch_freq_dist(const Geometry& geo, const double* w2, double cnst, double temp, int classical,
-                             double* freq, double* dist, int* err, cudaStream_t s) {
+                             double* freq, double* dist, double* occt, int* err, cudaStream_t s) {
   int n = geo.nkc * geo.b;
-  freq_dist_kernel<<<(n + 255) / 256, 256, 0, s>>>(geo, w2, cnst, temp, classical, freq, dist, err);
+  freq_dist_kernel<<<(n + 255) / 256, 256, 0, s>>>(geo, w2, cnst, temp, classical, freq, dist, occt, err);
   return cudaGetLastError();
 }
 

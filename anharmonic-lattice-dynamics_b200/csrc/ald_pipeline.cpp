@@ -190,7 +190,7 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   // the delta kernels read |V3|^2 slice by slice (coalesced over q2): the
   // class-form V3 kernels write that layout; the large-cell tensor-core V3
   // writes runs of l1 instead (layout 2)
-  const int v3_layout = v3_pipeline_layout(b, c->opt.precision);
+  const int v3_layout = capi::v3_layout(c);
   const bool mixed = c->opt.precision != ALD_FP64;
   const bool fused = !gauss && v3_layout != 2 && delta_fused_supported(c->geo);
   // deterministic option: the fused delta in two passes with fixed-point sums
@@ -198,13 +198,14 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   // of the chunk's R1/R2 (and R1p/R2p) size
   const bool det = fused && (c->opt.deterministic > 0 ||
                              (c->opt.deterministic == ALD_DET_AUTO && c->opt.precision == ALD_FP64));
-  // more than 16 bands, or layout 2: the band-generic delta kernels, straight into R1/R2
-  const bool any = !fused && (b > kDeltaSmallBands || v3_layout == 2);
+  // from 9 bands up the mixed V3 kernels write FP32
+  const bool v3_large_f32 = v3_layout == 2 || (mixed && v3_tile_used(c));
+  // more than 16 bands, or FP32 |V3|^2: the band-generic delta kernels, straight into R1/R2
+  const bool any = !fused && (b > kDeltaSmallBands || v3_large_f32);
   // the mixed pipeline hands |V3|^2 to the delta in FP32 where the delta
-  // reads it so: the large-cell tensor-core V3 (layout 2), and the class-form
-  // V3 of 3 and 6 bands into the fused tetrahedron delta.  Half the bytes,
-  // twice the rows per chunk.
-  const bool v3f = v3_layout == 2 || (mixed && fused && v3_layout == 1 && (b == 3 || b == 6));
+  // reads it so: from 9 bands up, and the class-form V3 of 3 and 6 bands into
+  // the fused tetrahedron delta.  Half the bytes, twice the rows per chunk.
+  const bool v3f = v3_large_f32 || (mixed && fused && v3_layout == 1 && (b == 3 || b == 6));
   int K = v3f ? std::min(nibz, 2 * rows_per_chunk(c)) : rows_per_chunk(c);
   const size_t v3n = (size_t)K * nkc * b * b * b;
   // where |V3|^2 takes several chunks it is not kept after the call, and a
@@ -257,6 +258,7 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
     a.v3sq_f32 = v3f ? reinterpret_cast<const float*>(v3.p) : nullptr;
     a.freq = c->freq.p;
     a.dist = c->dist.p;
+    a.occt = c->occt.p;
     a.tet_corner = c->tet_corner.p;
     a.tet_inc = c->tet_inc.p;
     a.gauss = gauss;
@@ -305,6 +307,9 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
       }
     } else if (fused) {
       ALD_CK(launch_delta_fused(a, s));
+      res->launches[2] += 1;
+    } else if (delta_gauss_pair_supported(a)) {
+      ALD_CK(launch_delta_gauss_pair(a, s));
       res->launches[2] += 1;
     } else if (any) {
       ALD_CK(launch_delta_any(a, s));

@@ -1044,6 +1044,74 @@ __global__ void __launch_bounds__(128) delta_gauss_any_kernel(CombineArgs a, con
   if (a.R2) a.R2[ri] = R[1];
 }
 
+// The pipeline's Gaussian delta from 6 bands up, |V3|^2 in layout 1
+// ([row][l2][l3][l1][q]): a thread takes q, l1, l2 and walks l3.  It reads each
+// |V3|^2(q) once, for process 1 at w = q and for process 2 at w = -q, whose q3
+// = q1 - w is the same point and whose |V3|^2 source is q again; omega and n
+// come band by band (occt), so every load of a warp (lanes = q) is a run.  A
+// CTA takes 32 q and 8 bands l2 of one l1 and sends R1 at q, R2 at -q out as
+// runs of 8 l2.  The Gaussian is delta_point_kernel's; (2 pi)^2/nkc, n1 and n2
+// are taken out of the sum over l3.  Bound by FP64 issue and the conversions
+// of the FP32 form.  Against a thread per (q, l1, l2) or (q, l2) that gathers
+// omega and n per point (delta_gauss_any_kernel, delta_point_kernel): 24 bands
+// 6x12x12 mixed 14.9 -> 7.2 ms, 48 bands 4x8x8 FP64 20.1 -> 10.5, 12 bands 8^3
+// FP64 1.31 -> 0.37, 6 bands 14^3 FP64 2.40 -> 1.56, mixed 1.14 -> 1.07.
+constexpr int kGpQ = 32, kGpL = 8;
+template <bool F32W, class VT>
+__global__ void __launch_bounds__(kGpQ* kGpL) delta_gauss_pair_kernel(CombineArgs a, const VT* __restrict__ v3sq) {
+  __shared__ double s_r[2][kGpQ][kGpL + 1];
+  __shared__ int s_wn[kGpQ];
+  const Geometry& g = a.geo;
+  const int b = g.b, nkc = g.nkc, b2 = b * b;
+  const int lane = threadIdx.x, nl2 = (b + kGpL - 1) / kGpL;
+  const int l1 = blockIdx.y / nl2, l20 = blockIdx.y % nl2 * kGpL, l2 = l20 + threadIdx.y, row = blockIdx.z;
+  const int q = blockIdx.x * kGpQ + lane;
+  const int q1 = a.mapinv[a.n1_first + row];
+  if (q < nkc && l2 < b) {
+    int m1[3], mq[3], m3[3], mn[3], ins;
+    decompose(g, q1, m1);
+    decompose(g, q, mq);
+    const int q3 = pm_index_m(g, m1, mq, 1, ins, m3);  // q1 + q = q1 - (-q)
+    for (int x = 0; x < 3; ++x) mn[x] = wrap2(-mq[x], g.nc[x]);
+    const int wn = compose(g, mn);
+    const bool g3 = at_gamma_index(g, m3);
+    const double* ft = a.occt;
+    const double* dt = a.occt + (size_t)nkc * b;
+    const double om1 = a.freq[(size_t)q1 * b + l1];
+    const double xa = om1 + ft[(size_t)l2 * nkc + q], xb = om1 - ft[(size_t)l2 * nkc + wn];
+    const double gc1 = 0.5 / (a.sigma * a.sigma), gc2 = 1.0 / (sqrt(2 * PhysConst::pi) * a.sigma);
+    const float fc1 = (float)gc1, fc2 = (float)gc2;
+    const VT* v = v3sq + (((size_t)row * b + l2) * b2 + l1) * nkc + q;
+    double r1 = 0.0, r2 = 0.0;
+#pragma unroll 4
+    for (int l3 = 0; l3 < b; ++l3) {
+      const double w3 = ft[(size_t)l3 * nkc + q3], n3 = dt[(size_t)l3 * nkc + q3] + 1;
+      const double vn = l3 < 3 && g3 ? 0.0 : (double)v[(size_t)l3 * b * nkc] * n3;
+      const double x1 = xa - w3, x2 = xb - w3;
+      if constexpr (F32W) {  // FP32 exp, underflows beyond 104
+        const float f1 = (float)x1, f2 = (float)x2, a1 = f1 * f1 * fc1, a2 = f2 * f2 * fc1;
+        if (a1 < 104.0f) r1 += (double)(expf(-a1) * fc2) * vn;
+        if (a2 < 104.0f) r2 += (double)(expf(-a2) * fc2) * vn;
+      } else {  // beyond 746
+        const double a1 = x1 * x1 * gc1, a2 = x2 * x2 * gc1;
+        if (a1 < 746.0) r1 += exp(-a1) * gc2 * vn;
+        if (a2 < 746.0) r2 += exp(-a2) * gc2 * vn;
+      }
+    }
+    const double n1f = a.dist[(size_t)q1 * b + l1] * ((2 * PhysConst::pi) * (2 * PhysConst::pi) / nkc);
+    s_r[0][lane][threadIdx.y] = l2 < 3 && at_gamma_index(g, mq) ? 0.0 : r1 * (n1f * dt[(size_t)l2 * nkc + q]);
+    s_r[1][lane][threadIdx.y] = l2 < 3 && at_gamma_index(g, mn) ? 0.0 : r2 * (n1f * (dt[(size_t)l2 * nkc + wn] + 1));
+    if (threadIdx.y == 0) s_wn[lane] = wn;
+  }
+  __syncthreads();
+  const int t = threadIdx.y * kGpQ + lane, k = t / kGpL, j = t % kGpL, qk = blockIdx.x * kGpQ + k;
+  if (qk < nkc && l20 + j < b) {
+    const size_t o = (size_t)l1 * b + l20 + j, r = (size_t)row * nkc;
+    a.R1[(r + qk) * b2 + o] = s_r[0][k][j];
+    a.R2[(r + s_wn[k]) * b2 + o] = s_r[1][k][j];
+  }
+}
+
 // Q, Q_N, Q_U of any number of bands: a CTA per (row, l1), threads over w
 __global__ void __launch_bounds__(256) q_from_r_any_kernel(Geometry g, int n1_first, const int* mapinv,
                                                            const double* R1, const double* R2, double* Q,
@@ -1256,6 +1324,23 @@ cudaError_t launch_delta_any(const CombineArgs& a, cudaStream_t s) {
       else delta_tet_any_kernel<false, double><<<grid, 256, smem, s>>>(a, a.v3sq);
     }
   }
+  return cudaGetLastError();
+}
+
+bool delta_gauss_pair_supported(const CombineArgs& a) {
+  const int nl2 = (a.geo.b + kGpL - 1) / kGpL;
+  return a.gauss && a.v3_layout == 1 && a.geo.b >= 6 && a.geo.b * nl2 <= 65535 && a.nrows <= 65535 && a.occt && a.R1 &&
+         a.R2 && !a.R1p && !a.R2p && !a.P1s && !a.P2s && !a.P1 && !a.P2;
+}
+
+cudaError_t launch_delta_gauss_pair(const CombineArgs& a, cudaStream_t s) {
+  if (!delta_gauss_pair_supported(a)) return cudaErrorInvalidValue;
+  const int b = a.geo.b;
+  const dim3 grid((a.geo.nkc + kGpQ - 1) / kGpQ, b * ((b + kGpL - 1) / kGpL), a.nrows), block(kGpQ, kGpL);
+  if (a.v3sq_f32 && a.f32w) delta_gauss_pair_kernel<true, float><<<grid, block, 0, s>>>(a, a.v3sq_f32);
+  else if (a.v3sq_f32) delta_gauss_pair_kernel<false, float><<<grid, block, 0, s>>>(a, a.v3sq_f32);
+  else if (a.f32w) delta_gauss_pair_kernel<true, double><<<grid, block, 0, s>>>(a, a.v3sq);
+  else delta_gauss_pair_kernel<false, double><<<grid, block, 0, s>>>(a, a.v3sq);
   return cudaGetLastError();
 }
 

@@ -31,6 +31,7 @@ SOURCES = {
     "ald_v3.cu": [],
     "ald_v3_pair.cu": [],
     "ald_v3_line.cu": [],
+    "ald_v3_tile.cu": [],
     "ald_v3_dense.cu": [],
     "ald_v3_dense_tc.cu": [],
     # weight_tet's FP32/FP64 arithmetic must not be contracted into FMAs
