@@ -204,6 +204,7 @@ int check_err_flags(ald_ctx* c) {
   CK(cudaStreamSynchronize(c->stream));
   if (h) {
     CK(cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
+    if (h & 64) c->det_overflow = true;  // no error: the pipeline runs again with the two-pass delta
     if (h & 16) return fail(ALD_ERR_CUDA, "V3: a tensor-core wait timed out (MMA completion not observed)");
     if (h & 32) return fail(ALD_ERR_CUDA, "eigensolver: the QL iteration did not converge in 60 sweeps");
     if (h & 2) return fail(ALD_ERR_DEN_ZERO, "MATRIX_ELT: den=0 (an eigenvalue is exactly zero)");

@@ -52,7 +52,10 @@ struct ald_ctx {
   DevBuf<double> w_brange;  // omega range of every band over the mesh
   DevBuf<char> w_scratch;
   DevBuf<double> w_heev;    // Householder eigensolver workspace (large cells)
-  DevBuf<double> w_rmax;    // deterministic delta: each R entry's largest term (FP64 bits)
+  DevBuf<double> w_rmax;    // deterministic delta: low parts of the sums, or each R entry's largest term (FP64 bits)
+  DevBuf<double> w_dscale;  // deterministic delta: its scales and bounds
+  bool det_overflow = false;  // a term was beyond the one-pass form's scale (check_err_flags)
+  bool det_two_pass = false;  // take the two-pass form
   // launch shapes chosen by ald_autotune (0 = the built-in choices)
   int tune_v3_rpc = 0, tune_v3_wg = 0;  // kept for ald_set_tuning's callers; nothing reads them
   size_t tune_gemm_bytes = 0;

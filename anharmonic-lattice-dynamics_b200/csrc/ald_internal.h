@@ -402,6 +402,11 @@ struct CombineArgs {
   unsigned long long* M2 = nullptr;
   unsigned long long* M1p = nullptr;
   unsigned long long* M2p = nullptr;
+  // the one-pass form (mode 3): M1/M2/M1p/M2p hold the low parts of the sums;
+  // scale: 2^S of (process, row, l1, l2), then of (process, row, l1, l3) with
+  // R1p/R2p; err: a term beyond the scale's headroom sets bit 64
+  const double* det_scale = nullptr;
+  int* err = nullptr;
   double* P1s;               // optional [row][q][l1][l2][l3] (P1smpi)
   double* P2s;
   double* P1;                // optional Bose-weighted
@@ -426,6 +431,14 @@ cudaError_t launch_combine(const CombineArgs& a, void* scratch, cudaStream_t s);
 bool delta_fused_supported(const Geometry& g);
 cudaError_t launch_delta_fused(const CombineArgs& a, cudaStream_t s, int mode = 0);
 cudaError_t launch_delta_finalize(double* R, const unsigned long long* M, size_t n, int b, cudaStream_t s);
+// mode 3, the same in one pass: launch_delta_scale bounds the terms of every
+// (process, row, l1, l2) from |V3|^2 and the Bose factors and forms
+// a.det_scale (work of delta_scale_doubles doubles, det_scale its first
+// part); mode 3 adds the terms in two integer parts of 2^-S and 2^-(S+52);
+// launch_delta_finalize_wide joins them.  R and M zero on entry.
+size_t delta_scale_doubles(int nrows, int b, bool marginals);
+cudaError_t launch_delta_scale(const CombineArgs& a, double* work, cudaStream_t s);
+cudaError_t launch_delta_finalize_wide(const CombineArgs& a, cudaStream_t s);
 // any number of bands (large cells): the tetrahedron or Gaussian delta into
 // R1/R2 and/or P1s/P2s straight from |V3|^2 of the chunk; for the tetrahedron
 // R1/R2/P1s/P2s (and R1p/R2p) must be zero on entry; P1/P2 are not produced

@@ -97,9 +97,8 @@ struct ShardSpec {
   void* user;
 };
 
-static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double* Qo, double* QNo, double* QUo,
-                        double* kappa_rta_modes, double* kappa_cg_modes, double* xo, const IterSpec* it,
-                        const ShardSpec* sh = nullptr) {
+static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, double* Qo, double* QNo, double* QUo,
+                        double* kappa_rta_modes, double* kappa_cg_modes, double* xo, const IterSpec* it, const ShardSpec* sh) {
   if (!c || !res) return fail(ALD_ERR_ARG, "null argument");
   if (sh && (sh->nranks < 1 || sh->rank < 0 || sh->rank >= sh->nranks || (!sh->gather && !sh->gather_dev)))
     return fail(ALD_ERR_ARG, "sharded pipeline: bad rank, rank count or exchange function");
@@ -193,15 +192,17 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   const int v3_layout = capi::v3_layout(c);
   const bool mixed = c->opt.precision != ALD_FP64;
   const bool fused = !gauss && v3_layout != 2 && delta_fused_supported(c->geo);
-  // deterministic option: the fused delta in two passes with fixed-point sums
-  // (the same bits on every run); its per-entry largest terms need a buffer
-  // of the chunk's R1/R2 (and R1p/R2p) size
+  // deterministic option: the fused delta with fixed-point sums (the same bits
+  // on every run); their low parts, or the two-pass form's largest terms, need
+  // a buffer of the chunk's R1/R2 (and R1p/R2p) size.  The one-pass form's rare
+  // second run is not for ranks that exchange: they keep to two passes
   const bool det = fused && (c->opt.deterministic > 0 ||
                              (c->opt.deterministic == ALD_DET_AUTO && c->opt.precision == ALD_FP64));
   // from 9 bands up the mixed V3 kernels write FP32
   const bool v3_large_f32 = v3_layout == 2 || (mixed && v3_tile_used(c));
   // more than 16 bands, or FP32 |V3|^2: the band-generic delta kernels, straight into R1/R2
   const bool any = !fused && (b > kDeltaSmallBands || v3_large_f32);
+  const bool wide = det && !sh && !c->det_two_pass;
   // the mixed pipeline hands |V3|^2 to the delta in FP32 where the delta
   // reads it so: from 9 bands up, and the class-form V3 of 3 and 6 bands into
   // the fused tetrahedron delta.  Half the bytes, twice the rows per chunk.
@@ -218,6 +219,7 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   if (!v3_gauss) ALD_CKA(v3.alloc(v3f ? (v3n + 1) / 2 : v3n));
   const size_t rchunk = (size_t)K * nkc * b * b;  // entries of one chunk's R1
   if (det) ALD_CKA(c->w_rmax.alloc((it ? 4 : 2) * rchunk));
+  if (wide) ALD_CKA(c->w_dscale.alloc(delta_scale_doubles(K, b, it != nullptr)));
   if (!fused && !any) ALD_CKA(escratch.alloc(std::max<size_t>(256, combine_scratch_bytes(c->geo, K, gauss))));
   ALD_CKA(c->w_brange.alloc((size_t)2 * b));
   ALD_CK(launch_band_range(c->geo, c->freq.p, c->w_brange.p, s));
@@ -293,6 +295,13 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
     if (v3_gauss) {
       r = run_v3_gauss(c, v3_args(c, r0, nr, nullptr), a, &res->launches[2]);
       if (r) return r;
+    } else if (wide) {
+      a.det_scale = c->w_dscale.p;
+      a.err = c->err.p;
+      ALD_CK(launch_delta_scale(a, c->w_dscale.p, s));
+      ALD_CK(launch_delta_fused(a, s, 3));
+      ALD_CK(launch_delta_finalize_wide(a, s));
+      res->launches[2] += it ? 7 : 5;
     } else if (det) {
       const size_t n = (size_t)nr * nkc * b * b;
       ALD_CK(launch_delta_fused(a, s, 1));
@@ -547,6 +556,21 @@ static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double*
   return ALD_OK;
 }
 
+// the one-pass deterministic delta found a term beyond its scale: once more
+// with the two-pass form (the flag does not depend on the order of the terms)
+static int run_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double* Qo, double* QNo, double* QUo,
+                        double* kappa_rta_modes, double* kappa_cg_modes, double* xo, const IterSpec* it,
+                        const ShardSpec* sh = nullptr) {
+  if (c) c->det_overflow = c->det_two_pass = false;
+  int r = run_pipeline_once(c, tempk, res, Qo, QNo, QUo, kappa_rta_modes, kappa_cg_modes, xo, it, sh);
+  if (c && c->det_overflow && r == ALD_OK) {
+    c->det_two_pass = true;
+    r = run_pipeline_once(c, tempk, res, Qo, QNo, QUo, kappa_rta_modes, kappa_cg_modes, xo, it, sh);
+    c->det_two_pass = false;
+  }
+  return r;
+}
+
 extern "C" int ald_kappa_pipeline(ald_ctx* c, double tempk, ald_kappa_result* res, double* Qo, double* QNo,
                                   double* QUo, double* kappa_rta_modes, double* kappa_cg_modes, double* xo) {
   return run_pipeline(c, tempk, res, Qo, QNo, QUo, kappa_rta_modes, kappa_cg_modes, xo, nullptr);
@@ -556,7 +580,7 @@ extern "C" int ald_kappa_pipeline(ald_ctx* c, double tempk, ald_kappa_result* re
 // device-memory cache, where the next structure of the same sizes finds them)
 static void release_pipeline_workspaces(ald_ctx* c) {
   c->v3c_epoch = 0;  // the kept |V3|^2 goes with its buffer
-  for (DevBuf<double>* b : {&c->w_R1, &c->w_R2, &c->w_v3, &c->w_cm, &c->w_R1p, &c->w_R2p, &c->w_heev, &c->w_rmax})
+  for (DevBuf<double>* b : {&c->w_R1, &c->w_R2, &c->w_v3, &c->w_cm, &c->w_R1p, &c->w_R2p, &c->w_heev, &c->w_rmax, &c->w_dscale})
     b->free();
   c->w_h.free();
   c->w_h64.free();

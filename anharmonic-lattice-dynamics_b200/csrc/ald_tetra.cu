@@ -452,15 +452,15 @@ __global__ void __launch_bounds__(256) q_from_r_kernel(Geometry g, int n1_first,
 // corners of those cells form a window of 2 x (R+1) x N2 mesh points.
 // Once per CTA the window's indices and flags are staged in shared memory;
 // then per l3 (one slice of the reference's loops):
-//   1. per window point: E = -+omega(w,l2) + omega(q1+-w,l3) as default REAL,
-//      G = n2 (n3+1) [process 1] or (n2+1)(n3+1) [process 2], G = 0 where the
-//      reference zeroes acoustic modes at Gamma (sub.f90:7351-7356, 7412-7417);
+//   1. per window point: E = -+omega(w,l2) + omega(q1+-w,l3) as default REAL;
 //   2. per cell: min/max of its 8 corner energies; cells whose range holds
 //      no band energy omega1(l1) are skipped, else its 6 tetrahedra are
 //      sorted once and each one whose range may hold an omega1(l1) is stored
 //      as a record (the window point at each sorted position; the energies
 //      are read back from the window) with its (record, l1) pairs queued;
-//   3. per queued pair: weight_tet's four corner weights c (bitwise, ald_tet.h)
+//   3. where pairs are queued, per window point: G = n2 (n3+1) [process 1] or
+//      (n2+1)(n3+1) [process 2], G = 0 where the reference zeroes acoustic
+//      modes at Gamma (sub.f90:7351-7356, 7412-7417); per queued pair: weight_tet's four corner weights c (bitwise, ald_tet.h)
 //      and R(row, w, l1, l2) += c/6 (2pi)^2/nkc |V3|^2 n1 G for each corner
 //      (FP64 atomics in L2; FP64 atomics on shared memory would be CAS loops).
 //      |V3|^2(src(w), l1, l2, l3) is gathered where needed; in the slice-major
@@ -476,6 +476,19 @@ __global__ void __launch_bounds__(256) q_from_r_kernel(Geometry g, int n1_first,
 // point, b slices l3 -- or b bands l2 for the marginals), so the sum stays
 // below 2^63 and each rounding is at most 2^-63 x 24 b of the entry.
 // launch_delta_finalize turns the integers back into doubles.
+//
+// MODE 3 (the deterministic option's usual form) needs no first pass: a term
+// is c |V3|^2 n1 G (2pi)^2/(6 nkc), and delta_bound_kernel takes the largest
+// |V3|^2 G of every (process, row, l1, l2) in one read of |V3|^2.  With that
+// bound and kDetCap for the corner weight c, S is chosen so that all kDetTerms
+// terms of an entry stay below 2^61 in units of 2^-S; a term is added as the
+// integer nearest to it in those units and the remainder in units of
+// 2^-(S+52), 113 bits below the bound in all.  The bound may therefore be
+// 2^50 above an entry's own sum before an FP64 sum would have been more exact.
+// A weight beyond kDetCap (a tetrahedron of energies within 1e-6 cm^-1 around
+// omega1) sets bit 64 of the error flag, and the pipeline takes MODE 1 and 2.
+// Rock-salt 16^3 FP64: 14.3 ms in two passes, 8.1 in one (B200; with the
+// queue's two ends, below).
 // corners of make_kp_reg_tet's six tetrahedra (c = o0 + 2 o1 + 4 o2), 3 bits
 // each, tetrahedra 0..4 in one word; tetrahedron 5 is (2, 5, 6, 7)
 constexpr unsigned long long kTetCornerCode =
@@ -501,6 +514,8 @@ __device__ __forceinline__ unsigned long long det_fixed(double v, unsigned long 
   return (unsigned long long)llrint(ldexp(v, 62 - det_exponent(m, b)));
 }
 
+constexpr double kDetCap = 4194304.0;  // 2^22, corner weights in 1/cm^-1
+
 struct FusedShape {
   int R, nbj, NW, maxrec;
   size_t smem;
@@ -524,11 +539,22 @@ __host__ __device__ inline FusedShape fused_shape(const Geometry& g) {
   return f;
 }
 
+// a term, scaled by 2^S, into the two integer parts of an entry; false when it
+// is beyond what S leaves room for
+__device__ __forceinline__ bool det_add(double t, int b, double* hi, unsigned long long* lo) {
+  if (!(t < 2305843009213693952.0 / kDetTerms(b))) return false;  // 2^61
+  const double h = rint(t);
+  atomicAdd(reinterpret_cast<unsigned long long*>(hi), (unsigned long long)(long long)h);
+  atomicAdd(lo, (unsigned long long)llrint((t - h) * 4503599627370496.0));  // 2^52
+  return true;
+}
+
 template <int B, bool F32W, class VT, int MODE>
 __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT* __restrict__ v3sq) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double s_om[B], s_nb1[B];
-  __shared__ int s_nrec, s_nq;
+  __shared__ double s_sc[MODE == 3 ? B : 1], s_scp[MODE == 3 ? B : 1];  // 2^S of R, R' per l1
+  __shared__ int s_nrec, s_nm, s_ne;  // records; queue entries from the front (mid) and from the back
   __shared__ unsigned short s_lp[kFusedThreads][8];              // window point of each cell corner
   __shared__ unsigned char s_hit[kFusedThreads / 32][32];      // the warp's cells that passed, by lane
   const Geometry& g = a.geo;
@@ -557,6 +583,7 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
   if (tid < b) {
     s_om[tid] = a.freq[(size_t)q1 * b + tid];
     s_nb1[tid] = a.dist[(size_t)q1 * b + tid];
+    if constexpr (MODE == 3) s_sc[tid] = a.det_scale[(((size_t)proc * a.nrows + row) * b + tid) * b + l2];
   }
   // conservative FP32 bounds of omega1 for the range tests (unused bands never count)
   float omlo[B], omhi[B];
@@ -602,6 +629,7 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
     sq = (size_t)b * b * b;
   }
   const VT* v3row = v3sq + (size_t)row * nkc * b * b * b;
+  const int qlast = maxrec * b - 1;  // the queue's last place
   // this thread's cell and its corners in the window
   const int cdj = tid / N2, ck = tid % N2;
   const bool cell_ok = tid < R * N2 && j0 + cdj < N1;
@@ -635,17 +663,13 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
   for (int l3 = 0; l3 < b; ++l3) {
     if (!((live >> l3) & 1u)) continue;
     __syncthreads();  // window staged / previous slice done
-    if (tid == 0) {
-      s_nrec = 0;
-      s_nq = 0;
-    }
+    if (tid == 0) s_nrec = s_nm = s_ne = 0;
+    if constexpr (MODE == 3)
+      if (Rpp && tid < b)
+        s_scp[tid] = a.det_scale[((((size_t)2 + proc) * a.nrows + row) * b + tid) * b + l3];
     for (int p = tid; p < NW; p += blockDim.x) {
-      const int q3 = s_q3[p];
-      const double fw = s_fw[p], f3 = a.freq[(size_t)q3 * b + l3];
+      const double fw = s_fw[p], f3 = a.occt[(size_t)l3 * nkc + s_q3[p]];
       s_E[p] = (float)(proc == 0 ? -fw + f3 : fw + f3);
-      const double n2 = s_n2[p], n3 = a.dist[(size_t)q3 * b + l3];
-      const bool zero = (l2 < 3 && (s_fl[p] & 1)) || (l3 < 3 && (s_fl[p] & 2));
-      s_G[p] = zero ? 0.0 : (proc == 0 ? n2 * (n3 + 1) : (n2 + 1) * (n3 + 1));
     }
     __syncthreads();
     // phase 1: cells -> tetrahedron records and (record, l1) pairs
@@ -705,7 +729,7 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
         int rbase = 0, qbase = 0;
         if (lane == 31 && incl != 0) {
           rbase = atomicAdd(&s_nrec, incl & 0xffff);
-          qbase = atomicAdd(&s_nq, incl >> 16);
+          qbase = atomicAdd(&s_nm, incl >> 16);
         }
         rbase = __shfl_sync(0xffffffffu, rbase, 31);
         qbase = __shfl_sync(0xffffffffu, qbase, 31);
@@ -739,7 +763,7 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
         const int nitem = 6 * __popc(hit);
         for (int it0 = 0; it0 < nitem; it0 += 32) {
           const int item = it0 + lane;
-          int cnt = 0, lo = 0;
+          int cnt = 0, lo = 0, m0 = 0, m1 = 0;
           float en[4];
           int cpt[4];
           if (item < nitem) {
@@ -753,47 +777,71 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
             }
             const float mn = fminf(fminf(en[0], en[1]), fminf(en[2], en[3]));
             const float mx = fmaxf(fmaxf(en[0], en[1]), fmaxf(en[2], en[3]));
+            // the two middle energies: min of the pairs' maxima, max of the pairs' minima
+            const float a1 = fmaxf(fminf(en[0], en[1]), fminf(en[2], en[3]));
+            const float a2 = fminf(fmaxf(en[0], en[1]), fmaxf(en[2], en[3]));
+            const float em = fminf(a1, a2), eM = fmaxf(a1, a2);
             int hi = 0;
   #pragma unroll
             for (int l1 = 0; l1 < B; ++l1) {
               lo += omhi[l1] < mn;
               hi += omlo[l1] <= mx;
+              m0 += omhi[l1] < em;
+              m1 += omlo[l1] <= eM;
             }
             cnt = hi > lo ? hi - lo : 0;
           }
-          const int packed = (cnt << 16) | (cnt > 0 ? 1 : 0);  // <= 32 records, <= 32*16 entries
-          int incl = packed;
+          const int nm = cnt > 0 ? max(m1 - m0, 0) : 0, ne = cnt - nm;
+          const unsigned packed = (unsigned)nm << 20 | (unsigned)ne << 8 | (cnt > 0 ? 1u : 0u);  // <= 32, <= 32*16
+          unsigned incl = packed;
   #pragma unroll
           for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
           }
-          int rbase = 0, qbase = 0;
+          int rbase = 0, mbase = 0, ebase = 0;
           if (lane == 31 && incl != 0) {
-            rbase = atomicAdd(&s_nrec, incl & 0xffff);
-            qbase = atomicAdd(&s_nq, incl >> 16);
+            rbase = atomicAdd(&s_nrec, (int)(incl & 0xffu));
+            mbase = atomicAdd(&s_nm, (int)(incl >> 20));
+            ebase = atomicAdd(&s_ne, (int)(incl >> 8 & 0xfffu));
           }
           rbase = __shfl_sync(0xffffffffu, rbase, 31);
-          qbase = __shfl_sync(0xffffffffu, qbase, 31);
+          mbase = __shfl_sync(0xffffffffu, mbase, 31);
+          ebase = __shfl_sync(0xffffffffu, ebase, 31);
           if (cnt > 0) {
-            const int rec = rbase + (incl & 0xffff) - 1;
-            int q = qbase + (incl >> 16) - cnt;
+            const int rec = rbase + (int)(incl & 0xffu) - 1;
+            int qm = mbase + (int)(incl >> 20) - nm, qe = qlast - (ebase + (int)(incl >> 8 & 0xfffu) - ne);
             // corner at each sorted position (tet_pos is a permutation of 0..3)
             const int ps0 = tet_pos(en, 0), ps1 = tet_pos(en, 1), ps2 = tet_pos(en, 2);
             auto at = [&](int p) {
               return (unsigned short)(ps0 == p ? cpt[0] : ps1 == p ? cpt[1] : ps2 == p ? cpt[2] : cpt[3]);
             };
             s_recp[rec] = make_ushort4(at(0), at(1), at(2), at(3));
-            for (int l1 = lo; l1 < lo + cnt; ++l1) s_queue[q++] = (unsigned short)((rec << 4) | l1);
+            for (int l1 = lo; l1 < lo + cnt; ++l1)
+              s_queue[l1 >= m0 && l1 < m1 ? qm++ : qe--] = (unsigned short)((rec << 4) | l1);
           }
         }
       }
     }
     __syncthreads();
-    // phase 2: corner weights of the queued pairs into R
-    const int nq = s_nq;
-    for (int i = tid; i < nq; i += blockDim.x) {
-      const unsigned v = s_queue[i];
+    // phase 2: corner weights of the queued pairs into R.  FP64: the pairs with
+    // omega1 between the tetrahedron's middle energies stand at the queue's
+    // front and the others at its back, and no warp takes both: weight_tet's
+    // middle branch has three times the divisions of the others, and a warp
+    // pays for every branch that one of its lanes takes.  (Mixed: the weights
+    // are cheap, and the second queue cost more than it gave: 3.58 ms against
+    // 3.19 at 16^3.)
+    const int nm = s_nm, ne = F32W ? 0 : s_ne, nmw = F32W ? nm : (nm + 31) & ~31;
+    if (nm + ne == 0) continue;  // the same for every thread
+    for (int p = tid; p < NW; p += blockDim.x) {
+      const double n2 = s_n2[p], n3 = a.occt[(size_t)(b + l3) * nkc + s_q3[p]];
+      const bool zero = (l2 < 3 && (s_fl[p] & 1)) || (l3 < 3 && (s_fl[p] & 2));
+      s_G[p] = zero ? 0.0 : (proc == 0 ? n2 * (n3 + 1) : (n2 + 1) * (n3 + 1));
+    }
+    __syncthreads();
+    for (int i = tid; i < nmw + ne; i += blockDim.x) {
+      if (i >= nm && i < nmw) continue;
+      const unsigned v = s_queue[i < nm ? i : qlast - (i - nmw)];
       const int rec = (int)(v >> 4), l1 = (int)(v & 15u);
       const ushort4 pp = s_recp[rec];
       // sorted positions 0..3 hold the highest .. lowest corner
@@ -825,6 +873,10 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
           const unsigned long long bits = (unsigned long long)__double_as_longlong(val);
           atomicMax(Mp + o + w, bits);
           if (Rpp) atomicMax(Mpp + op + w, bits);
+        } else if constexpr (MODE == 3) {
+          if (!det_add(val * s_sc[l1], b, Rp + o + w, Mp + o + w) ||
+              (Rpp && !det_add(val * s_scp[l1], b, Rpp + op + w, Mpp + op + w)))
+            atomicOr(a.err, 64);
         } else {
           atomicAdd(reinterpret_cast<unsigned long long*>(Rp + o + w), det_fixed(val, Mp[o + w], b));
           if (Rpp) atomicAdd(reinterpret_cast<unsigned long long*>(Rpp + op + w), det_fixed(val, Mpp[op + w], b));
@@ -853,6 +905,90 @@ __global__ void delta_finalize_kernel(double* R, const unsigned long long* __res
     const unsigned long long m = M[i];
     const unsigned long long acc = reinterpret_cast<const unsigned long long*>(R)[i];
     R[i] = m == 0 ? 0.0 : ldexp((double)acc, det_exponent(m, b) - 62);
+  }
+}
+
+// A bound of |V3|^2 G for every (process, row, l1, l2) -- and (process, row,
+// l1, l3) for the marginals -- as FP64 bits, at most 2^-20 above the largest
+// (a maximum does not depend on the order).  A CTA takes one slice (l2, l3) of one row; every
+// |V3|^2(q) serves process 1 at w = q and process 2 at w = -q.  One read of
+// |V3|^2, coalesced over q in the slice-major layout.
+template <int B, class VT>
+__global__ void __launch_bounds__(256) delta_bound_kernel(CombineArgs a, const VT* __restrict__ v3sq,
+                                                          unsigned long long* bnd) {
+  const Geometry& g = a.geo;
+  const int b = g.b, nkc = g.nkc, b2 = b * b, row = blockIdx.y;
+  const int l2 = blockIdx.x / b, l3 = blockIdx.x % b;
+  const int q1 = a.mapinv[a.n1_first + row];
+  int m1[3];
+  decompose(g, q1, m1);
+  const size_t sq = a.v3_layout == 1 ? 1 : (size_t)b2 * b, s1 = a.v3_layout == 1 ? (size_t)nkc : (size_t)b2;
+  const VT* v = v3sq + (size_t)row * nkc * b2 * b +
+                (a.v3_layout == 1 ? ((size_t)l2 * b + l3) * b * nkc : (size_t)l2 * b + l3);
+  const double* dt = a.occt + (size_t)nkc * b;
+  // the high words of nonnegative doubles order as the doubles do; one more
+  // than the largest, with a zero low word, bounds them all
+  int mx1[B], mx2[B];
+#pragma unroll
+  for (int l = 0; l < B; ++l) mx1[l] = mx2[l] = 0;
+#pragma unroll 2
+  for (int q = threadIdx.x; q < nkc; q += blockDim.x) {
+    int mq[3], m3[3], mn[3], ins;
+    decompose(g, q, mq);
+    const int q3 = pm_index_m(g, m1, mq, 1, ins, m3);
+    for (int x = 0; x < 3; ++x) mn[x] = wrap2(-mq[x], g.nc[x]);
+    const int wn = compose(g, mn);
+    const double n3 = l3 < 3 && at_gamma_index(g, m3) ? 0.0 : dt[(size_t)l3 * nkc + q3] + 1;
+    const double g1 = l2 < 3 && at_gamma_index(g, mq) ? 0.0 : dt[(size_t)l2 * nkc + q] * n3;
+    const double g2 = l2 < 3 && at_gamma_index(g, mn) ? 0.0 : (dt[(size_t)l2 * nkc + wn] + 1) * n3;
+#pragma unroll
+    for (int l = 0; l < B; ++l) {
+      if (l >= b) continue;
+      const double x = (double)v[(size_t)q * sq + l * s1];
+      mx1[l] = max(mx1[l], __double2hiint(x * g1));
+      mx2[l] = max(mx2[l], __double2hiint(x * g2));
+    }
+  }
+  const size_t nr = (size_t)a.nrows * b2;
+#pragma unroll
+  for (int l = 0; l < B; ++l) {
+    if (l >= b) continue;
+    const int h1 = __reduce_max_sync(0xffffffffu, mx1[l]), h2 = __reduce_max_sync(0xffffffffu, mx2[l]);
+    if ((threadIdx.x & 31) == 0) {
+      const unsigned long long x1 = (unsigned long long)(h1 + 1) << 32, x2 = (unsigned long long)(h2 + 1) << 32;
+      const size_t r = ((size_t)row * b + l) * b;
+      atomicMax(bnd + r + l2, x1);
+      atomicMax(bnd + nr + r + l2, x2);
+      if (a.R1p) {
+        atomicMax(bnd + 2 * nr + r + l3, x1);
+        atomicMax(bnd + 3 * nr + r + l3, x2);
+      }
+    }
+  }
+}
+
+// 2^S of every bound: kDetTerms terms of at most bound n1 (2pi)^2/(6 nkc)
+// kDetCap stay below 2^61 (S within +-1000)
+__global__ void delta_scale_kernel(CombineArgs a, const unsigned long long* bnd, double* scale, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const Geometry& g = a.geo;
+  const int b = g.b, l1 = i / b % b, row = i / (b * b) % a.nrows;
+  const double n1 = a.dist[(size_t)a.mapinv[a.n1_first + row] * b + l1];
+  const double fnorm6 = (2 * PhysConst::pi) * (2 * PhysConst::pi) / g.nkc / 6.0;
+  int e;
+  frexp(__longlong_as_double((long long)bnd[i]) * fnorm6 * n1 * (kDetCap * kDetTerms(b)), &e);
+  scale[i] = ldexp(1.0, max(-1000, min(1000, 61 - e)));
+}
+
+// the two integer parts of MODE 3 joined, in place
+__global__ void delta_finalize_wide_kernel(double* R, const unsigned long long* __restrict__ L,
+                                           const double* __restrict__ scale, size_t n, int nkc, int b) {
+  const size_t b2 = (size_t)b * b;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+    const long long hi = reinterpret_cast<const long long*>(R)[i], lo = (long long)L[i];
+    const size_t row = i / (b2 * nkc);
+    R[i] = ((double)hi + (double)lo * 2.220446049250313e-16) / scale[row * b2 + i % b2];  // 2^-52
   }
 }
 
@@ -1286,6 +1422,7 @@ cudaError_t launch_delta_fused(const CombineArgs& a, cudaStream_t s, int mode) {
   if (!a.M1 || !a.M2 || (a.R1p && !a.M1p) || (a.R2p && !a.M2p)) return cudaErrorInvalidValue;
   if (mode == 1) return launch_delta_fused_mode<1>(a, s);
   if (mode == 2) return launch_delta_fused_mode<2>(a, s);
+  if (mode == 3 && a.det_scale && a.err) return launch_delta_fused_mode<3>(a, s);
   return cudaErrorInvalidValue;
 }
 
@@ -1293,6 +1430,48 @@ cudaError_t launch_delta_finalize(double* R, const unsigned long long* M, size_t
   if (n == 0) return cudaSuccess;
   const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
   delta_finalize_kernel<<<blocks, 256, 0, s>>>(R, M, n, b);
+  return cudaGetLastError();
+}
+
+size_t delta_scale_doubles(int nrows, int b, bool marginals) {
+  return (size_t)2 * (marginals ? 4 : 2) * nrows * b * b;  // scales, then bounds
+}
+
+cudaError_t launch_delta_scale(const CombineArgs& a, double* work, cudaStream_t s) {
+  const int b = a.geo.b, n = (a.R1p ? 4 : 2) * a.nrows * b * b;
+  unsigned long long* bnd = reinterpret_cast<unsigned long long*>(work + n);
+  cudaError_t e = cudaMemsetAsync(bnd, 0, (size_t)n * sizeof(double), s);
+  if (e != cudaSuccess) return e;
+  const dim3 grid(b * b, a.nrows);
+#define ALD_BOUND(BB)                                                                 \
+  if (a.v3sq_f32) delta_bound_kernel<BB><<<grid, 256, 0, s>>>(a, a.v3sq_f32, bnd);     \
+  else delta_bound_kernel<BB><<<grid, 256, 0, s>>>(a, a.v3sq, bnd);
+  if (b <= 3) {
+    ALD_BOUND(3)
+  } else if (b <= 6) {
+    ALD_BOUND(6)
+  } else if (b <= 12) {
+    ALD_BOUND(12)
+  } else if (b <= kMaxBandsTet) {
+    ALD_BOUND(16)
+  } else {
+    return cudaErrorInvalidValue;
+  }
+#undef ALD_BOUND
+  delta_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(a, bnd, work, n);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_delta_finalize_wide(const CombineArgs& a, cudaStream_t s) {
+  const int b = a.geo.b, nkc = a.geo.nkc;
+  const size_t n = (size_t)a.nrows * nkc * b * b, nr = (size_t)a.nrows * b * b;
+  const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
+  delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R1, a.M1, a.det_scale, n, nkc, b);
+  delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R2, a.M2, a.det_scale + nr, n, nkc, b);
+  if (a.R1p) {
+    delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R1p, a.M1p, a.det_scale + 2 * nr, n, nkc, b);
+    delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R2p, a.M2p, a.det_scale + 3 * nr, n, nkc, b);
+  }
   return cudaGetLastError();
 }
 

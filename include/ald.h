@@ -66,8 +66,8 @@ typedef struct ald_options {
   int device;        /* CUDA device ordinal                                             */
   size_t chunk_bytes;/* device bytes for one chunk of |V3|^2 rows (0 = automatic)      */
   int deterministic; /* the pipeline's tetrahedron delta (up to 16 bands):
-                        1: sums with the same bits on every run (two passes, the second
-                        with fixed-point integer atomics; about 2.4x the delta's time),
+                        1: sums with the same bits on every run (fixed-point integer
+                        atomics; about 1.4x the delta's time),
                         0: FP64 atomics in arrival order (last bits vary between runs),
                         ALD_DET_AUTO (-1, the default): 1 for ALD_FP64, 0 otherwise    */
 } ald_options;
