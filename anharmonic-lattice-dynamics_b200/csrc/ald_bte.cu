@@ -314,8 +314,13 @@ __global__ void ffull_kernel(Geometry g, const int* mapibz, const int* full_op, 
 // part[row][slice][l1][xyz].
 constexpr int kUpdSlices = 8;
 
-__global__ void update_partial_kernel(Geometry g, int n1_first, const int* mapinv, const double* R1, const double* R1p,
-                                      const double* R2, const double* R2p, const double* Ff, double* part) {
+__global__ void __launch_bounds__(256) update_partial_kernel(Geometry g, int n1_first, const int* mapinv,
+                                                             const double* __restrict__ R1,
+                                                             const double* __restrict__ R1p,
+                                                             const double* __restrict__ R2,
+                                                             const double* __restrict__ R2p,
+                                                             const double* __restrict__ Ff,
+                                                             const int4* __restrict__ mesh_m, double* part) {
   __shared__ double red[256][3];
   const int b = g.b, b2 = b * b, nkc = g.nkc;
   const int nl = blockIdx.y, sl = blockIdx.x;
@@ -323,15 +328,20 @@ __global__ void update_partial_kernel(Geometry g, int n1_first, const int* mapin
   int m1[3];
   decompose(g, q1, m1);
   const int t = threadIdx.x, l = t % b;  // l1 = (t / b) % b
-  const size_t e0 = (size_t)(sl * nkc / kUpdSlices) * b2, e1 = (size_t)((sl + 1) * nkc / kUpdSlices) * b2;
-  const size_t rb = (size_t)nl * nkc * b2;
+  const int step = blockDim.x / b2, qend = (sl + 1) * nkc / kUpdSlices;
+  const size_t rb = (size_t)nl * nkc * b2 + t % b2;
   double a0 = 0, a1 = 0, a2 = 0;
-  for (size_t e = e0 + t; e < e1; e += blockDim.x) {
-    const int q = (int)(e / b2);
-    int mq[3], ins;
-    decompose(g, q, mq);
+  // unrolled so that the marginals of several q are in flight; the mesh
+  // integers from the table instead of divisions (rock-salt 12^3: 136 -> 94 us
+  // per iteration against 41 us for the marginals at the copy bandwidth)
+#pragma unroll 4
+  for (int q = sl * nkc / kUpdSlices + t / b2; q < qend; q += step) {
+    const int4 mm = __ldg(mesh_m + q);
+    const int mq[3] = {mm.x, mm.y, mm.z};
+    int ins;
     const int qp = pm_index(g, m1, mq, 1, ins), qm = pm_index(g, m1, mq, -1, ins);
-    const double c1 = R1[rb + e], c1p = R1p[rb + e], c2 = R2[rb + e], c2p = R2p[rb + e];
+    const size_t e = rb + (size_t)q * b2;
+    const double c1 = R1[e], c1p = R1p[e], c2 = R2[e], c2p = R2p[e];
     const double* fq = Ff + ((size_t)q * b + l) * 3;
     const double* fp = Ff + ((size_t)qp * b + l) * 3;
     const double* fm = Ff + ((size_t)qm * b + l) * 3;
@@ -346,8 +356,8 @@ __global__ void update_partial_kernel(Geometry g, int n1_first, const int* mapin
   if (t < 3 * b) {
     const int L1 = t / 3, x = t % 3;
     double A = 0;
-    for (int u = 0; u < (int)blockDim.x; ++u)
-      if ((u / b) % b == L1) A += red[u][x];
+    for (int u = L1 * b; u < (int)blockDim.x; u += b2)
+      for (int j = 0; j < b; ++j) A += red[u + j][x];
     part[(((size_t)nl * kUpdSlices + sl) * b + L1) * 3 + x] = A;
   }
 }
@@ -666,12 +676,13 @@ size_t update_part_doubles(const Geometry& geo, int nrows) { return (size_t)nrow
 cudaError_t launch_update(const Geometry& geo, int n1_first, int nrows, const int* mapinv, const double* R1,
                           const double* R1p, const double* R2, const double* R2p, const double* Ff, const double* Q,
                           const double* F_RTA, const double* F, double mix, double* Fout, double* part,
-                          cudaStream_t s) {
+                          const int* mesh_m, cudaStream_t s) {
   const int b2 = geo.b * geo.b;
   if (b2 > 256) return cudaErrorInvalidValue;
   const int threads = b2 * (256 / b2);
   dim3 grid(kUpdSlices, nrows);
-  update_partial_kernel<<<grid, threads, 0, s>>>(geo, n1_first, mapinv, R1, R1p, R2, R2p, Ff, part);
+  update_partial_kernel<<<grid, threads, 0, s>>>(geo, n1_first, mapinv, R1, R1p, R2, R2p, Ff,
+                                                  reinterpret_cast<const int4*>(mesh_m), part);
   const int n = nrows * geo.b * 3;
   update_final_kernel<<<(n + 255) / 256, 256, 0, s>>>(geo, n1_first, nrows, part, Q, F_RTA, F, mix, Fout);
   return cudaGetLastError();

@@ -546,6 +546,13 @@ int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
     a.hbuf = c->w_h.p;
     e = launch_v3_line(a, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
     nl += 4;  // mode factors, class sums H, plane sums, the line kernel
+  } else if (v3_pair_lines_supported(c->geo, v3_line_tables(c))) {
+    // 6 bands: class sums axis by axis, mode products per pair
+    const int r = v3_line_alloc(c, a.nrows);
+    if (r) return r;
+    a.hbuf = c->w_h.p;
+    e = launch_v3_pair_lines(a, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
+    nl += 3;
   } else if (v3_pair_supported(c->geo.b, prec)) {
     const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, a.nrows, prec);
     if (c->w_h.n < need) CKA(c->w_h.alloc(need));
@@ -742,7 +749,7 @@ int ald_create_from_dir(const char* dir, const ald_options* opt, ald_ctx** out) 
       }
     }
     st.add(c->roots, rt);
-    if (c->S.include_fc[2] == 1 && c->T.b == 3) {
+    if (c->S.include_fc[2] == 1 && (c->T.b == 3 || c->T.b == 6)) {
       V3Lines& ln = c->VL;
       build_v3_lines(c->S, c->T, c->VC, rt, ln);
       st.add(c->ln_cls, ln.cls);
@@ -1336,7 +1343,7 @@ int ald_update_mpi(ald_ctx* c, const int ksubset[2], const double* P1, const dou
   CK(cudaMemcpyAsync(f.p, hf.data(), nf * sizeof(double), cudaMemcpyHostToDevice, s));
   CK(launch_ffull(c->geo, c->mapibz0.p, c->full_op.p, c->opk.p, f.p, ff.p, s));
   CK(launch_update(c->geo, ksubset[0] - 1, nr, c->mapinv.p, R1.p, R1p.p, R2.p, R2p.p, ff.p, q.p, frta.p, f.p, 0.0,
-                   out.p, part.p, s));
+                   out.p, part.p, c->mesh_m.p, s));
   std::vector<double> ho((size_t)nr * b * 3);
   CK(cudaMemcpyAsync(ho.data(), out.p, ho.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
   CK(cudaStreamSynchronize(s));

@@ -322,9 +322,7 @@ struct V3Args {
   long long npairs_list = 0;
 };
 cudaError_t launch_v3_fp64(const V3Args& a, cudaStream_t s);
-// 3 and 6 bands, class sums axis by axis (ald_v3_line.cu): V3Lines on the
-// device; hbuf of v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) bytes and work of
-// v3_line_work_bytes (per-mode factors, the row's sums per mesh line)
+// V3Lines on the device
 struct V3LineTables {
   int ns2, ns3;
   const int* cls;
@@ -335,6 +333,8 @@ struct V3LineTables {
   const double* ph1;
   const double* ph2;
 };
+// 3 bands, class sums axis by axis (ald_v3_line.cu): hbuf of v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) bytes and work of
+// v3_line_work_bytes (per-mode factors, the row's sums per mesh line)
 bool v3_line_supported(const Geometry& g, const V3LineTables& t, int precision);
 size_t v3_line_row_bytes(const Geometry& g, const V3LineTables& t, int precision);
 size_t v3_line_work_bytes(const Geometry& g, const V3LineTables& t, int nrows, int precision);
@@ -343,6 +343,15 @@ cudaError_t launch_v3_line(const V3Args& a, const V3LineTables& t, void* work, i
 bool v3_pair_supported(int b, int precision);
 size_t v3_hbuf_bytes(int b, int ncls, int nrows, int precision);
 cudaError_t launch_v3_pair(const V3Args& a, int precision, cudaStream_t s);
+// the same with the class sums taken from the row's sums per mesh line
+// (6 bands); hbuf of v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) bytes, work of
+// v3_line_work_bytes
+bool v3_pair_lines_supported(const Geometry& g, const V3LineTables& t);
+cudaError_t launch_v3_pair_lines(const V3Args& a, const V3LineTables& t, void* work, int precision, cudaStream_t s);
+// steps 1 and 2 of ald_v3_line.cu alone: H in a.hbuf (FP64) to the line sums,
+// [row][line][slot 3][be ga][l1] complex (3 bands: [l1][be ga])
+cudaError_t launch_v3_lines(const V3Args& a, const V3LineTables& t, void* lines, int precision, cudaStream_t s);
+bool v3_lines_supported(const Geometry& g, const V3LineTables& t);
 // row stage alone, H in FP32 or FP64
 cudaError_t launch_v3_rows_f32(const V3Args& a, cudaStream_t s);
 cudaError_t launch_v3_rows_f64(const V3Args& a, cudaStream_t s);
@@ -537,7 +546,7 @@ cudaError_t launch_ffull(const Geometry& geo, const int* mapibz, const int* full
 size_t update_part_doubles(const Geometry& geo, int nrows);
 cudaError_t launch_update(const Geometry& geo, int n1_first, int nrows, const int* mapinv, const double* R1,
                           const double* R1p, const double* R2, const double* R2p, const double* Ff, const double* Q,
-                          const double* F_RTA, const double* F, double mix, double* Fout, double* part,
+                          const double* F_RTA, const double* F, double mix, double* Fout, double* part, const int* mesh_m,
                           cudaStream_t s);
 // CG workspace: vectors, scalars and the captured CUDA graph of the
 // iteration loop, kept across calls and re-captured only when the problem

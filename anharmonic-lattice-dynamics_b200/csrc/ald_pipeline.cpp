@@ -395,7 +395,7 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
     for (int i = 1; i <= it->max_iter; ++i) {
       ALD_CK(launch_ffull(c->geo, c->mapibz0.p, c->full_op.p, c->opk.p, F.p, Ff.p, s));
       ALD_CK(launch_update(c->geo, 0, nibz, c->mapinv.p, R1.p, c->w_R1p.p, R2.p, c->w_R2p.p, Ff.p, dQ, Frta.p, F.p,
-                           it->mix, F.p, c->w_part.p, s));
+                           it->mix, F.p, c->w_part.p, c->mesh_m.p, s));
       ALD_CK(launch_kappa(k, F.p, 0, kc.p, c->err.p, s));
       res->launches[7] += 3;
       ALD_CK(cudaMemcpyAsync(knew.data(), kc.p, knew.size() * sizeof(double), cudaMemcpyDeviceToHost, s));

@@ -117,28 +117,29 @@ __global__ void v3_line_modes_kernel(const double* __restrict__ w2, const double
 // runs.  About a sixth of the line kernel's time (argon 26^3, 299 rows: 0.22
 // of 1.23 ms); bound by the phase and H2 loads.
 constexpr int kPlaneThreads = 256, kPlaneM = 4;
-template <class C>
+template <class C, int COMPS>
 __global__ void __launch_bounds__(kPlaneThreads) v3_plane_kernel(V3Args a, V3LineTables t, C* __restrict__ H3) {
   extern __shared__ __align__(16) unsigned char smraw[];
-  double2* H2 = reinterpret_cast<double2*>(smraw);  // [slot 2][27]
+  double2* H2 = reinterpret_cast<double2*>(smraw);  // [slot 2][component]
   const int m0 = blockIdx.x, row = blockIdx.y;
   const int N0 = a.geo.nc[0], N1 = a.geo.nc[1], ns3 = t.ns3;
-  const double2* H = static_cast<const double2*>(a.hbuf) + (size_t)row * a.ncls * 27;
+  const double2* H = static_cast<const double2*>(a.hbuf) + (size_t)row * a.ncls * COMPS;
   const double2* ph0 = reinterpret_cast<const double2*>(t.ph0) + (size_t)m0 * a.ncls;
   const double2* ph1 = reinterpret_cast<const double2*>(t.ph1);
-  for (int e = threadIdx.x; e < t.ns2 * 27; e += kPlaneThreads) {
-    const int s = e / 27, k = e - s * 27;
+  for (int e = threadIdx.x; e < t.ns2 * COMPS; e += kPlaneThreads) {
+    const int s = e / COMPS, k = e - s * COMPS;
     double2 acc = make_double2(0.0, 0.0);
-    for (int c = t.s2_off[s]; c < t.s2_off[s + 1]; ++c) cmac(acc, ph0[c], H[(size_t)t.cls[c] * 27 + k]);
-    H2[s * 27 + k] = acc;
+    for (int c = t.s2_off[s]; c < t.s2_off[s + 1]; ++c) cmac(acc, ph0[c], H[(size_t)t.cls[c] * COMPS + k]);
+    H2[s * COMPS + k] = acc;
   }
   __syncthreads();
-  // a thread takes kPlaneM values of m_1 and the components k, k + 9, k + 18:
+  // a thread takes kPlaneM values of m_1 and the components k, k + COMPS/3, k + 2 COMPS/3:
   // 4 phases and 3 sums loaded for 12 products
-  C* out = H3 + ((size_t)row * N0 + m0) * N1 * ns3 * 27;
+  C* out = H3 + ((size_t)row * N0 + m0) * N1 * ns3 * COMPS;
+  constexpr int K3 = COMPS / 3;
   const int nm = (N1 + kPlaneM - 1) / kPlaneM;
-  for (int e = threadIdx.x; e < nm * ns3 * 9; e += kPlaneThreads) {
-    const int ms = e / 9, k = e - ms * 9, mb = ms / ns3, s = ms - mb * ns3;
+  for (int e = threadIdx.x; e < nm * ns3 * K3; e += kPlaneThreads) {
+    const int ms = e / K3, k = e - ms * K3, mb = ms / ns3, s = ms - mb * ns3;
     const double2* p[kPlaneM];
     double2 acc[kPlaneM][3];
 #pragma unroll
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kPlaneThreads) v3_plane_kernel(V3Args a, V3Lin
     for (int c = t.s3_off[s]; c < t.s3_off[s + 1]; ++c) {
       double2 h[3];
 #pragma unroll
-      for (int j = 0; j < 3; ++j) h[j] = H2[c * 27 + k + 9 * j];
+      for (int j = 0; j < 3; ++j) h[j] = H2[c * COMPS + k + K3 * j];
 #pragma unroll
       for (int i = 0; i < kPlaneM; ++i) {
         const double2 ph = p[i][c];
@@ -161,11 +162,11 @@ __global__ void __launch_bounds__(kPlaneThreads) v3_plane_kernel(V3Args a, V3Lin
 #pragma unroll
     for (int i = 0; i < kPlaneM; ++i) {
       if (mb * kPlaneM + i >= N1) continue;
-      C* o = out + ((size_t)(mb * kPlaneM + i) * ns3 + s) * 27;
+      C* o = out + ((size_t)(mb * kPlaneM + i) * ns3 + s) * COMPS;
 #pragma unroll
-      for (int j = 0; j < 3; ++j) {  // [be ga][l1] -> [l1][be ga]
-        const int kj = k + 9 * j;
-        o[kj % 3 * 9 + kj / 3] = cvt<C>(acc[i][j]);
+      for (int j = 0; j < 3; ++j) {
+        const int kj = k + K3 * j;  // [be ga][l1]; 3 bands: to [l1][be ga]
+        o[COMPS == 27 ? kj % 3 * 9 + kj / 3 : kj] = cvt<C>(acc[i][j]);
       }
     }
   }
@@ -349,8 +350,17 @@ size_t line_smem(const Geometry& g, int ns3) {
 }
 // the work buffer: 1/sqrt|lambda| and the FP32 eigenvectors of the mesh, then H3
 size_t line_align(size_t x) { return (x + 255) / 256 * 256; }
-size_t line_t_bytes(const Geometry& g) { return line_align((size_t)g.nkc * 3 * sizeof(double)); }
-size_t line_e_bytes(const Geometry& g) { return line_align((size_t)g.nkc * 9 * sizeof(float2)); }
+size_t line_t_bytes(const Geometry& g) { return line_align((size_t)g.nkc * g.b * sizeof(double)); }
+size_t line_e_bytes(const Geometry& g) { return line_align((size_t)g.nkc * g.b * g.b * sizeof(float2)); }
+
+template <class C, int COMPS>
+cudaError_t launch_plane_t(const V3Args& a, const V3LineTables& t, void* lines, cudaStream_t s) {
+  const size_t smem = (size_t)t.ns2 * COMPS * sizeof(double2);
+  const cudaError_t e = raise_smem_limit((const void*)v3_plane_kernel<C, COMPS>, smem);
+  if (e != cudaSuccess) return e;
+  v3_plane_kernel<C, COMPS><<<dim3(a.geo.nc[0], a.nrows), kPlaneThreads, smem, s>>>(a, t, static_cast<C*>(lines));
+  return cudaGetLastError();
+}
 
 template <class T>
 cudaError_t launch_line_t(const V3Args& a, const V3LineTables& t, void* work, const LineGauss* d, cudaStream_t s) {
@@ -364,10 +374,8 @@ cudaError_t launch_line_t(const V3Args& a, const V3LineTables& t, void* work, co
   v3_line_modes_kernel<<<(g.nkc * 3 + 255) / 256, 256, 0, s>>>(a.w2, ev, g.nkc * 3, ts, ef);
   cudaError_t e = launch_v3_rows_f64(a, s);
   if (e != cudaSuccess) return e;
-  const size_t psm = (size_t)t.ns2 * 27 * sizeof(double2);
-  e = raise_smem_limit((const void*)v3_plane_kernel<C>, psm);
+  e = launch_v3_lines(a, t, H3, sizeof(T) == 4 ? ALD_MIXED : ALD_FP64, s);
   if (e != cudaSuccess) return e;
-  v3_plane_kernel<C><<<dim3(g.nc[0], a.nrows), kPlaneThreads, psm, s>>>(a, t, H3);
   const size_t smem = line_smem<T>(g, t.ns3);
   LineModes<T> md;
   md.t = ts;
@@ -388,14 +396,25 @@ cudaError_t launch_line_t(const V3Args& a, const V3LineTables& t, void* work, co
 
 }  // namespace
 
+bool v3_lines_supported(const Geometry& g, const V3LineTables& t) {
+  return (g.b == 3 || g.b == 6) && t.ns2 >= 1 && (size_t)t.ns2 * 9 * g.b * sizeof(double2) <= 200 * 1024;
+}
+
+cudaError_t launch_v3_lines(const V3Args& a, const V3LineTables& t, void* lines, int precision, cudaStream_t s) {
+  if (!v3_lines_supported(a.geo, t)) return cudaErrorInvalidValue;
+  if (precision == ALD_FP64)
+    return a.geo.b == 3 ? launch_plane_t<double2, 27>(a, t, lines, s) : launch_plane_t<double2, 54>(a, t, lines, s);
+  return a.geo.b == 3 ? launch_plane_t<float2, 27>(a, t, lines, s) : launch_plane_t<float2, 54>(a, t, lines, s);
+}
+
 bool v3_line_supported(const Geometry& g, const V3LineTables& t, int precision) {
-  if (g.b != 3 || t.ns2 < 1 || (size_t)t.ns2 * 27 * sizeof(double2) > 200 * 1024) return false;
+  if (g.b != 3 || !v3_lines_supported(g, t)) return false;
   return (precision == ALD_FP64 ? line_smem<double>(g, t.ns3) : line_smem<float>(g, t.ns3)) <= 200 * 1024;
 }
 
 size_t v3_line_row_bytes(const Geometry& g, const V3LineTables& t, int precision) {
   const size_t cplx = precision == ALD_FP64 ? sizeof(double2) : sizeof(float2);
-  return (size_t)g.nc[0] * g.nc[1] * t.ns3 * 27 * cplx;
+  return (size_t)g.nc[0] * g.nc[1] * t.ns3 * 9 * g.b * cplx;
 }
 
 size_t v3_line_work_bytes(const Geometry& g, const V3LineTables& t, int nrows, int precision) {

@@ -129,8 +129,14 @@ __global__ void v3_row_kernel(V3Args a) {
 // Tasks: class sums (q, j0 be, k0 ga) -> B values of l1 each;
 // mode product 2 (q, c', l1 block) -> (B/S) x B accumulators;
 // mode product 3 (q, l1, l2 block) -> (B/S) x B accumulators and |V|^2.
-template <class T, int B, int QT, int S, int NT>
-__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) v3_pair_kernel(V3Args a) {
+// LINES: the class sums from the row's sums per mesh line (ald_v3_line.cu): one
+// term per slot 3 of the group -- 3 each for rock-salt, against 13 or 6 classes
+// -- whose phase goes by m_2 alone.  Lanes walk q, so that most read one line.
+// Rock-salt 16^3, V3 stage: FP64 3.65 -> 2.81 ms, mixed 1.99 -> 1.80 (B200);
+// FP64 now bound by shared memory (the e(q2), e(q3) reads of the products).
+template <class T, int B, int QT, int S, int NT, bool LINES>
+__global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2)
+    v3_pair_kernel(V3Args a, V3LineTables lt, const typename Cx<T>::t* __restrict__ lines) {
   using C = typename Cx<T>::t;
   constexpr int NAT = B / 3, B2 = B * B, B3 = B2 * B, NG = NAT * NAT;
   constexpr int AP = B3 | 1, EP = B2 | 1, BS = B / S;
@@ -138,7 +144,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) v3_pair_kernel(V3A
   C* sm = reinterpret_cast<C*>(smraw);
   const Geometry& g = a.geo;
   const int tid = threadIdx.x, row = blockIdx.y;
-  const int PP = a.ncls | 1;
+  const int PP = (LINES ? lt.ns3 : a.ncls) | 1;
   C* At = sm;
   C* E2 = At + QT * AP;
   C* E3 = E2 + QT * EP;
@@ -172,7 +178,14 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) v3_pair_kernel(V3A
     E3[q * EP + e] = cvt<C>(ev[(size_t)s_q3[q] * B2 + e]);
   }
   const double2* roots = reinterpret_cast<const double2*>(a.roots);
-  for (int i = tid; i < QT * a.ncls; i += NT) {
+  if constexpr (LINES) {
+    const double2* ph2 = reinterpret_cast<const double2*>(lt.ph2);
+    for (int i = tid; i < QT * lt.ns3; i += NT) {
+      const int q = i % QT, s = i / QT;
+      P[q * PP + s] = cvt<C>(ph2[(size_t)(s_q2[q] % g.nc[2]) * lt.ns3 + s]);
+    }
+  }
+  for (int i = tid; !LINES && i < QT * a.ncls; i += NT) {
     const int q = i % QT, c = i / QT;
     int m2[3];
     decompose(g, s_q2[q], m2);
@@ -184,7 +197,7 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) v3_pair_kernel(V3A
   // q + QT/2), so that each H value it loads serves two pairs (FP64: one q,
   // the registers of two would spill)
   const C* H = static_cast<const C*>(a.hbuf) + (size_t)row * a.ncls * 9 * B;
-  constexpr int QB = sizeof(T) == 4 ? 2 : 1, QH = QT / QB;
+  constexpr int QB = sizeof(T) == 4 && !LINES ? 2 : 1, QH = QT / QB;
   for (int task = tid; task < QH * NG * 9; task += NT) {
     const int q = task % QH, col = task / QH;
     const int grp = col / 9, bg = col % 9;
@@ -194,7 +207,17 @@ __global__ void __launch_bounds__(NT, sizeof(T) == 4 ? 3 : 2) v3_pair_kernel(V3A
     for (int k = 0; k < QB; ++k)
 #pragma unroll
       for (int l = 0; l < B; ++l) acc[k][l] = C{0, 0};
-    const int c0 = a.cls_grp_off[grp], c1 = a.cls_grp_off[grp + 1];
+    if constexpr (LINES) {
+      const C* hl = lines + (((size_t)row * g.nc[0] * g.nc[1] + s_q2[q] / g.nc[2]) * lt.ns3 * 9 + bg) * B;
+      const int s1 = lt.grp_off[grp + 1];
+      for (int s = lt.grp_off[grp]; s < s1; ++s) {
+        const C p = P[q * PP + s];
+        const C* h = hl + s * 9 * B;
+#pragma unroll
+        for (int l = 0; l < B; ++l) cmac(acc[0][l], p, h[l]);
+      }
+    }
+    const int c0 = LINES ? 0 : a.cls_grp_off[grp], c1 = LINES ? 0 : a.cls_grp_off[grp + 1];
     for (int c = c0; c < c1; ++c) {
       C p[QB];
 #pragma unroll
@@ -303,22 +326,27 @@ struct PairCfg {
   int qt, nt;
 };
 
-template <class T, int B, int QT, int S, int NT>
-cudaError_t launch_pair_t(const V3Args& a, cudaStream_t s) {
+template <class T, int B, int QT, int S, int NT, bool LINES>
+cudaError_t launch_pair_k(const V3Args& a, const V3LineTables& t, const void* lines, cudaStream_t s) {
   using C = typename Cx<T>::t;
   constexpr int B2 = B * B, B3 = B2 * B;
-  const size_t smem = ((size_t)QT * ((B3 | 1) + 2 * (B2 | 1) + (a.ncls | 1))) * sizeof(C);
+  const size_t smem = ((size_t)QT * ((B3 | 1) + 2 * (B2 | 1) + ((LINES ? t.ns3 : a.ncls) | 1))) * sizeof(C);
   if (smem > 220 * 1024) return cudaErrorInvalidValue;
-  cudaError_t e = raise_smem_limit((const void*)v3_pair_kernel<T, B, QT, S, NT>, smem);
+  cudaError_t e = raise_smem_limit((const void*)v3_pair_kernel<T, B, QT, S, NT, LINES>, smem);
   if (e != cudaSuccess) return e;
+  dim3 grid((a.geo.nkc + QT - 1) / QT, a.nrows);
+  v3_pair_kernel<T, B, QT, S, NT, LINES><<<grid, NT, smem, s>>>(a, t, static_cast<const C*>(lines));
+  return cudaGetLastError();
+}
+
+template <class T, int B, int QT, int S, int NT>
+cudaError_t launch_pair_t(const V3Args& a, cudaStream_t s) {
   // row stage
   const int n = a.ncls * 9 * B;
   dim3 rg((n + 255) / 256, a.nrows);
-  v3_row_kernel<C><<<rg, 256, 0, s>>>(a);
+  v3_row_kernel<typename Cx<T>::t><<<rg, 256, 0, s>>>(a);
   // pair stage
-  dim3 grid((a.geo.nkc + QT - 1) / QT, a.nrows);
-  v3_pair_kernel<T, B, QT, S, NT><<<grid, NT, smem, s>>>(a);
-  return cudaGetLastError();
+  return launch_pair_k<T, B, QT, S, NT, false>(a, V3LineTables(), nullptr, s);
 }
 
 }  // namespace
@@ -357,6 +385,19 @@ cudaError_t launch_v3_pair(const V3Args& a, int precision, cudaStream_t s) {
     if (b == 6) return launch_pair_t<double, 6, 16, 3, 288>(a, s);
   }
   return cudaErrorInvalidValue;
+}
+
+bool v3_pair_lines_supported(const Geometry& g, const V3LineTables& t) {
+  return g.b == 6 && v3_lines_supported(g, t) && t.ns3 <= 256;  // phases beside A, e2, e3 in shared memory
+}
+
+cudaError_t launch_v3_pair_lines(const V3Args& a, const V3LineTables& t, void* work, int precision, cudaStream_t s) {
+  if (!v3_pair_lines_supported(a.geo, t)) return cudaErrorInvalidValue;
+  cudaError_t e = launch_v3_rows_f64(a, s);
+  if (e == cudaSuccess) e = launch_v3_lines(a, t, work, precision, s);
+  if (e != cudaSuccess) return e;
+  return precision != ALD_FP64 ? launch_pair_k<float, 6, 16, 3, 288, true>(a, t, work, s)
+                               : launch_pair_k<double, 6, 16, 3, 288, true>(a, t, work, s);
 }
 
 }  // namespace ald
