@@ -518,7 +518,7 @@ int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
       CKA(c->w_v3work.alloc(wb));
       zeroed = false;
     }
-    e = launch_v3_rows_f32(a, c->stream);
+    e = launch_v3_rows_by_class_f32(a, c->stream);
     if (e == cudaSuccess) e = launch_v3_dense_tc(a, c->w_v3work.p, P, zeroed, c->stream);
     c->v3work_tc_b = e == cudaSuccess ? c->geo.b : 0;
     c->v3work_tc_p = P;

@@ -366,7 +366,7 @@ cudaError_t launch_v3_dense(const V3Args& a, void* work, size_t work_bytes, cuda
 // `row` of the chunk of a, in a's layout and precision, bands l1 < l1_keep
 cudaError_t launch_v3_copy_row(const V3Args& a, int row, const double* src, int l1_keep, cudaStream_t s);
 // more than 6 bands, ALD_MIXED (ald_v3_dense_tc.cu): both mode products as
-// split-FP16 tcgen05 GEMMs; hbuf from launch_v3_rows_f32; work of
+// split-FP16 tcgen05 GEMMs; hbuf from launch_v3_rows_by_class_f32; work of
 // v3_dense_tc_work_bytes(b, nkc, nrows, pairs) bytes for batches of `pairs`
 // pairs; a2_zeroed: the workspace's T2 operand padding is already zero
 bool v3_dense_tc_supported(int b);
@@ -384,6 +384,8 @@ int v3_pipeline_layout(int b, int precision);
 bool v3_tile_supported(const Geometry& g, int ncls, int precision);
 size_t v3_tile_work_bytes(const Geometry& g, int ncls, int nrows, int precision);
 cudaError_t launch_v3_tile(const V3Args& a, void* work, int precision, cudaStream_t s, int l1_keep = 0);
+// its row stage alone, in FP32 into a.hbuf: H[row][c][l1][be ga]
+cudaError_t launch_v3_rows_by_class_f32(const V3Args& a, cudaStream_t s);
 struct CombineArgs {
   Geometry geo;
   int n1_first, nrows;

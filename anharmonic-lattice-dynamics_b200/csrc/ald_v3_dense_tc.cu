@@ -203,10 +203,10 @@ __global__ void v3tc_rowbound_kernel(V3Args a, unsigned* bound) {
   const long long n = (long long)nat0 * nat0 * 9 * b;
   float mx = 0.f;
   for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-    const int l1 = (int)(e % b), bg = (int)((e / b) % 9), grp = (int)(e / (9LL * b));
+    const int bg = (int)(e % 9), l1 = (int)((e / 9) % b), grp = (int)(e / (9LL * b));
     float sm = 0.f;
     for (int c = a.cls_grp_off[grp]; c < a.cls_grp_off[grp + 1]; ++c) {
-      const float2 h = H[((size_t)c * 9 + bg) * b + l1];
+      const float2 h = H[((size_t)c * b + l1) * 9 + bg];
       sm += fabsf(h.x) + fabsf(h.y);
     }
     mx = fmaxf(mx, sm);
@@ -232,7 +232,12 @@ __global__ void v3tc_rowexp_kernel(int nrows, const unsigned* bound, int* rexp) 
 }
 
 // A operand of GEMM 1 for the batch's pairs: rows m = l1 b + kc, K' = (Re |
-// Im) jb; a thread per (row of the tile, K group of 8 jb)
+// Im) jb; a thread per (row of the tile, 24 jb = 8 atoms j0 = 3 K groups of
+// 8), so that one look at a group's classes -- most of a large cell's groups
+// have none -- serves its three be.  H is [row][c][l1][be ga]: the be and ga of
+// one class are one run.  Bound by the operand's 16-byte stores and the H reads
+// (192 bands: one jb at a time with H [c][be ga][l1] took 43 us per pair).
+constexpr int kT1J = 8;  // atoms j0 per thread
 __global__ void __launch_bounds__(256) v3tc_t1_kernel(V3Args a, DenseTc t, long long pair0, int table_ph) {
   extern __shared__ float2 s_ph[];  // P_c(q2) of every class
   const DenseTcShape& s = t.sh;
@@ -253,38 +258,50 @@ __global__ void __launch_bounds__(256) v3tc_t1_kernel(V3Args a, DenseTc t, long 
   const float2* H = static_cast<const float2*>(a.hbuf) + (size_t)pi.row * a.ncls * 9 * b;
   const float sc = ldexpf(1.f, kSplitE - t.rexp[pi.row]);
   __half* A = t.a1 + (size_t)p * s.a_pair_halves;
-  const int ng = s.kh / 8;
-  for (int e = threadIdx.x; e < kTM * ng; e += blockDim.x) {
-    const int r = e % kTM, kg = e / kTM, m = mt * kTM + r;
-    float xr[8], xi[8];
+  const int ng = s.kh / 8, nj = (ng + 2) / 3;
+  for (int e = threadIdx.x; e < kTM * nj; e += blockDim.x) {
+    const int r = e % kTM, jg = e / kTM, m = mt * kTM + r;
+    float xr[3 * kT1J], xi[3 * kT1J];
     const bool live = m < b * b;
     const int l1 = live ? m / b : 0, kc = live ? m % b : 0, k0 = kc / 3, ga = kc % 3;
+    const float2* hl = H + (size_t)l1 * 9 + ga;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int jb = kg * 8 + i;
-      float2 acc = make_float2(0.f, 0.f);
-      if (live && jb < b) {
-        const int grp = (jb / 3) * nat0 + k0, be = jb % 3;
-        for (int c = a.cls_grp_off[grp]; c < a.cls_grp_off[grp + 1]; ++c) {
+    for (int j = 0; j < kT1J; ++j) {
+      const int j0 = jg * kT1J + j;
+      float2 acc[3] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+      if (live && j0 < nat0) {
+        const int grp = j0 * nat0 + k0, c1 = __ldg(a.cls_grp_off + grp + 1);
+        for (int c = __ldg(a.cls_grp_off + grp); c < c1; ++c) {
           float2 ph;
           if (table_ph) {
             ph = s_ph[c];
           } else {
-            const double2 r = roots[phase_index(a.cls_pc + 4 * c, m2, g.L, g.L32)];
-            ph = make_float2((float)r.x, (float)r.y);
+            const double2 z = roots[phase_index(a.cls_pc + 4 * c, m2, g.L, g.L32)];
+            ph = make_float2((float)z.x, (float)z.y);
           }
-          const float2 h = H[((size_t)c * 9 + be * 3 + ga) * b + l1];
-          acc.x = fmaf(ph.x, h.x, fmaf(-ph.y, h.y, acc.x));
-          acc.y = fmaf(ph.x, h.y, fmaf(ph.y, h.x, acc.y));
+#pragma unroll
+          for (int be = 0; be < 3; ++be) {
+            const float2 h = hl[(size_t)c * b * 9 + be * 3];
+            acc[be].x = fmaf(ph.x, h.x, fmaf(-ph.y, h.y, acc[be].x));
+            acc[be].y = fmaf(ph.x, h.y, fmaf(ph.y, h.x, acc[be].y));
+          }
         }
       }
-      xr[i] = acc.x * sc;
-      xi[i] = acc.y * sc;
+#pragma unroll
+      for (int be = 0; be < 3; ++be) {
+        xr[3 * j + be] = acc[be].x * sc;
+        xi[3 * j + be] = acc[be].y * sc;
+      }
     }
-    __half* hr = A + a_group_off(s, m, kg);
-    split8(xr, hr, hr + (size_t)kTM * kBK);
-    __half* him = A + a_group_off(s, m, s.kh / 8 + kg);
-    split8(xi, him, him + (size_t)kTM * kBK);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const int kg = 3 * jg + k;
+      if (kg >= ng) continue;
+      __half* hr = A + a_group_off(s, m, kg);
+      split8(xr + 8 * k, hr, hr + (size_t)kTM * kBK);
+      __half* him = A + a_group_off(s, m, ng + kg);
+      split8(xi + 8 * k, him, him + (size_t)kTM * kBK);
+    }
   }
 }
 

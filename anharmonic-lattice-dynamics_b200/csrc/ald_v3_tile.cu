@@ -421,6 +421,12 @@ bool v3_tile_supported(const Geometry& g, int ncls, int precision) {
   return precision == ALD_FP64 ? tile_shape<double>(g, ncls, s) : tile_shape<float>(g, ncls, s);
 }
 
+cudaError_t launch_v3_rows_by_class_f32(const V3Args& a, cudaStream_t s) {
+  v3_tile_row_kernel<float2><<<dim3((a.ncls * 9 * a.geo.b + 255) / 256, a.nrows), 256, 0, s>>>(
+      a, static_cast<float2*>(a.hbuf));
+  return cudaGetLastError();
+}
+
 size_t v3_tile_work_bytes(const Geometry& g, int ncls, int nrows, int precision) {
   const size_t cplx = precision == ALD_FP64 ? sizeof(double2) : sizeof(float2);
   return tile_align((size_t)g.nkc * g.b * sizeof(double)) + (size_t)nrows * ncls * 9 * g.b * cplx;
