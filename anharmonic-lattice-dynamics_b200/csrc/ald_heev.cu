@@ -23,10 +23,16 @@
 // point need eigenvalues only: no Z, no V.
 //
 // Work per matrix: tridiagonalisation (4/3) b^3 complex multiply-adds, each
-// step a warp-per-row matrix-vector product and a rank-2 update of the
+// step a matrix-vector product (four rows per warp) and a rank-2 update of the
 // trailing block; QL: the rotations of a sweep are formed by one thread
-// (a serial recurrence) and applied to the rows of Z by all threads; the
-// back-transformation b^3 complex multiply-adds, one eigenvector per thread.
+// (a serial recurrence) while the other warps apply the sweep before it to the
+// rows of Z; the back-transformation b^3 complex multiply-adds, one eigenvector
+// per thread.  448 matrices of 192 bands on B200: 38 -> 32 ms, in SM cycles per
+// matrix 23 M tridiagonalisation (memory: three passes over the trailing block
+// per step, all matrices together exceed L2), 28 M QL (the chain of a hypot, a
+// quotient and their products per rotation), 8 M back-transformation; the two
+// exchange sorts by one thread took as long before equal values were the only
+// ones left to them.
 // The QL loop is bounded: 60 sweeps per eigenvalue, after which bit 5 of the
 // error flag is set.
 #include <cuda_runtime.h>
@@ -143,17 +149,47 @@ __device__ void he_dynmat(const PhononArgs& a, const double* q, double2* A, doub
   __syncthreads();
 }
 
+// the exchange sort's order of x[0..b): where no two values are equal every
+// sort gives it, and a value's place is the number of smaller ones
+__device__ void he_order(const double* x, int* ord, int b, int* tie) {
+  if (threadIdx.x == 0) *tie = 0;
+  __syncthreads();
+  for (int i = threadIdx.x; i < b; i += blockDim.x) {
+    int n = 0, eq = 0;
+    for (int j = 0; j < b; ++j) {
+      n += x[j] < x[i];
+      eq += !(x[j] < x[i]) && !(x[j] > x[i]);  // itself, an equal value or a NaN
+    }
+    if (eq > 1) *tie = 1;
+    else ord[n] = i;
+  }
+  __syncthreads();
+  if (*tie && threadIdx.x == 0) {
+    for (int i = 0; i < b; ++i) ord[i] = i;
+    for (int i = 0; i < b; ++i)
+      for (int j = i + 1; j < b; ++j)
+        if (x[ord[i]] > x[ord[j]]) {
+          const int t = ord[i];
+          ord[i] = ord[j];
+          ord[j] = t;
+        }
+  }
+  __syncthreads();
+}
+
+constexpr int kHeRows = 4;
+
 struct HeShared {
   double2 v[kHeMaxB];      // Householder vector of the current step
   double2 p[kHeMaxB];      // A v, then w
   double2 dl[kHeMaxB];     // diagonal phases of the real tridiagonal form
   double d[kHeMaxB], e[kHeMaxB], tau[kHeMaxB];
-  double rc[kHeMaxB], rs[kHeMaxB];  // rotations of one QL sweep
+  double rc[2][kHeMaxB], rs[2][kHeMaxB];  // rotations of two QL sweeps
   double lab[kHeMaxB];
   int ord[kHeMaxB], ord2[kHeMaxB];
   double red[kHeThreads / 32];
   double2 kred[kHeThreads / 32];
-  int cmd, lo, hi;
+  int cmd, lo[2], hi[2], tie;
 };
 
 __host__ __device__ inline size_t heev_slot_doubles(int b) {
@@ -161,7 +197,10 @@ __host__ __device__ inline size_t heev_slot_doubles(int b) {
   return 5 * bb + (bb & 1);
 }
 
-__global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat) {
+// MINB CTAs per SM: 2 leave the compiler 128 registers, 4 hold it to 64 and let
+// more matrices hide each other's serial QL (launch_heev's rule)
+template <int MINB>
+__global__ void __launch_bounds__(kHeThreads, MINB) heev_kernel(PhononArgs a, int nmat) {
   __shared__ HeShared S;
   const int b = a.geo.b, bb = b * b;
   const int tid = threadIdx.x, nth = blockDim.x, warp = tid >> 5, lane = tid & 31, nwarp = nth >> 5;
@@ -172,7 +211,8 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
   double2* V = A + bb;
   double* Z = slot + (size_t)4 * bb;
   for (int mat = blockIdx.x; mat < nmat; mat += gridDim.x) {
-    const int pt = mat / a.ndisp, dsp = mat % a.ndisp;
+    // the points' own matrices, which also need eigenvectors, first
+    const int npt = nmat / a.ndisp, pt = mat % npt, dsp = mat / npt;
     const bool vecs = dsp == 0;
     double q[3] = {a.kpc32[3 * pt], a.kpc32[3 * pt + 1], a.kpc32[3 * pt + 2]};
     if (dsp > 0) {
@@ -217,20 +257,35 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
         S.dl[k] = make_double2(-ph.x * nrm, -ph.y * nrm);  // eps_k, turned into a phase below
       }
       __syncthreads();
-      // p = tau A22 v: one warp per row, lanes over the columns
-      for (int i = warp; i < m; i += nwarp) {
-        const double2* Ar = A + (size_t)(k + 1 + i) * b + (k + 1);
-        double2 s = make_double2(0.0, 0.0);
+      // p = tau A22 v: a warp takes kHeRows rows at a time, lanes over the
+      // columns, so that the rows' loads overlap
+      for (int i0 = warp * kHeRows; i0 < m; i0 += nwarp * kHeRows) {
+        const double2* Ar[kHeRows];
+        double2 s[kHeRows];
+#pragma unroll
+        for (int r = 0; r < kHeRows; ++r) {
+          Ar[r] = A + (size_t)(k + 1 + min(i0 + r, m - 1)) * b + (k + 1);
+          s[r] = make_double2(0.0, 0.0);
+        }
         for (int j = lane; j < m; j += 32) {
-          const double2 x = Ar[j], v = S.v[j];
-          s.x = fma(x.x, v.x, fma(-x.y, v.y, s.x));
-          s.y = fma(x.x, v.y, fma(x.y, v.x, s.y));
+          const double2 v = S.v[j];
+          double2 x[kHeRows];
+#pragma unroll
+          for (int r = 0; r < kHeRows; ++r) x[r] = Ar[r][j];
+#pragma unroll
+          for (int r = 0; r < kHeRows; ++r) {
+            s[r].x = fma(x[r].x, v.x, fma(-x[r].y, v.y, s[r].x));
+            s[r].y = fma(x[r].x, v.y, fma(x[r].y, v.x, s[r].y));
+          }
         }
-        for (int o = 16; o > 0; o >>= 1) {
-          s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
-          s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+#pragma unroll
+        for (int r = 0; r < kHeRows; ++r) {
+          for (int o = 16; o > 0; o >>= 1) {
+            s[r].x += __shfl_xor_sync(0xffffffffu, s[r].x, o);
+            s[r].y += __shfl_xor_sync(0xffffffffu, s[r].y, o);
+          }
+          if (lane == 0 && i0 + r < m) S.p[i0 + r] = make_double2(tau * s[r].x, tau * s[r].y);
         }
-        if (lane == 0) S.p[i] = make_double2(tau * s.x, tau * s.y);
       }
       __syncthreads();
       // K = (tau/2) v^H p
@@ -260,13 +315,27 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
       }
       __syncthreads();
       // A22 -= v w^H + w v^H
-      for (size_t e = tid; e < (size_t)m * m; e += nth) {
-        const int i = (int)(e / m), j = (int)(e % m);
-        const double2 vi = S.v[i], wi = S.p[i], vj = S.v[j], wj = S.p[j];
-        const double2 t1 = cmul(vi, cconj(wj)), t2 = cmul(wi, cconj(vj));
-        double2* x = A + (size_t)(k + 1 + i) * b + (k + 1 + j);
-        const double2 o = *x;
-        *x = make_double2(o.x - t1.x - t2.x, o.y - t1.y - t2.y);
+      for (int i0 = warp * kHeRows; i0 < m; i0 += nwarp * kHeRows) {
+        double2 vi[kHeRows], wi[kHeRows];
+#pragma unroll
+        for (int r = 0; r < kHeRows; ++r) {
+          vi[r] = S.v[min(i0 + r, m - 1)];
+          wi[r] = S.p[min(i0 + r, m - 1)];
+        }
+        for (int j = lane; j < m; j += 32) {
+          const double2 vj = S.v[j], wj = S.p[j];
+          double2* x = A + (size_t)(k + 1 + i0) * b + (k + 1 + j);
+          double2 o[kHeRows];
+#pragma unroll
+          for (int r = 0; r < kHeRows; ++r)
+            if (i0 + r < m) o[r] = x[(size_t)r * b];
+#pragma unroll
+          for (int r = 0; r < kHeRows; ++r) {
+            if (i0 + r >= m) continue;
+            const double2 t1 = cmul(vi[r], cconj(wj)), t2 = cmul(wi[r], cconj(vj));
+            x[(size_t)r * b] = make_double2(o[r].x - t1.x - t2.x, o[r].y - t1.y - t2.y);
+          }
+        }
       }
       __syncthreads();
     }
@@ -294,10 +363,13 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
       for (size_t e = tid; e < (size_t)bb; e += nth) Z[e] = (e / b == e % b) ? 1.0 : 0.0;
     __syncthreads();
     // ---------------------------------------------------------- implicit QL
-    // thread 0 forms the rotations of one sweep (e[i] couples i and i+1);
-    // every thread then applies them, in order, to its rows of Z
+    // thread 0 forms the rotations of one sweep (e[i] couples i and i+1); the
+    // threads of the other warps meanwhile apply the sweep before it, in order,
+    // to their rows of Z (they do not touch d and e)
     int ql_l = 0, ql_iter = 0;
-    for (;;) {
+    for (int sw = 0;; ++sw) {
+      double* const rc = S.rc[sw & 1];
+      double* const rs = S.rs[sw & 1];
       if (tid == 0) {
         int cmd = 1;  // done
         while (ql_l < b) {
@@ -340,62 +412,62 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
             p = s * r;
             S.d[i + 1] = g + p;
             g = c * r - bq;
-            S.rc[i] = c;
-            S.rs[i] = s;
+            rc[i] = c;
+            rs[i] = s;
           }
           if (!under) {
             S.d[l] -= p;
             S.e[l] = g;
             S.e[m] = 0.0;
           }
-          S.hi = m - 1;
-          S.lo = under ? i + 1 : l;
+          S.hi[sw & 1] = m - 1;
+          S.lo[sw & 1] = under ? i + 1 : l;
           cmd = 0;
           break;
         }
         S.cmd = cmd;
+      } else if (vecs && warp > 0 && sw > 0) {
+        // the lower row of one rotation is the upper row of the next: carried
+        // in a register, and eight rows loaded ahead
+        const double* pc = S.rc[(sw - 1) & 1];
+        const double* ps = S.rs[(sw - 1) & 1];
+        const int hi = S.hi[(sw - 1) & 1], lo = S.lo[(sw - 1) & 1];
+        for (int rr = tid - 32; rr < b; rr += nth - 32) {
+          if (hi < lo) continue;
+          double f = Z[(size_t)(hi + 1) * b + rr];
+          int i = hi;
+          for (; i - 7 >= lo; i -= 8) {
+            double z[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) z[j] = Z[(size_t)(i - j) * b + rr];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              const double c = pc[i - j], s = ps[i - j];
+              Z[(size_t)(i - j + 1) * b + rr] = s * z[j] + c * f;
+              f = c * z[j] - s * f;
+            }
+          }
+          for (; i >= lo; --i) {
+            const double c = pc[i], s = ps[i], z = Z[(size_t)i * b + rr];
+            Z[(size_t)(i + 1) * b + rr] = s * z + c * f;
+            f = c * z - s * f;
+          }
+          Z[(size_t)lo * b + rr] = f;
+        }
       }
       __syncthreads();
       const int cmd = S.cmd;
+      __syncthreads();  // cmd read before thread 0 writes the next one
       if (cmd != 0) break;
-      if (vecs) {
-        const int hi = S.hi, lo = S.lo;
-        for (int rr = tid; rr < b; rr += nth)
-          for (int i = hi; i >= lo; --i) {
-            const double c = S.rc[i], s = S.rs[i];
-            const double f = Z[(size_t)(i + 1) * b + rr], z = Z[(size_t)i * b + rr];
-            Z[(size_t)(i + 1) * b + rr] = s * z + c * f;
-            Z[(size_t)i * b + rr] = c * z - s * f;
-          }
-      }
-      __syncthreads();
     }
     // ---------------------------------------------------------- ordering
     // get_freq: ascending signed eigenvalues (exchange sort of
     // extratools.f90:154-175), eival = |lambda|; get_frequencies sorts the
     // |lambda| once more (velocities keep the first order)
-    if (tid == 0) {
-      for (int i = 0; i < b; ++i) S.ord[i] = i;
-      for (int i = 0; i < b; ++i)
-        for (int j = i + 1; j < b; ++j)
-          if (S.d[S.ord[i]] > S.d[S.ord[j]]) {
-            const int t = S.ord[i];
-            S.ord[i] = S.ord[j];
-            S.ord[j] = t;
-          }
-      for (int i = 0; i < b; ++i) {
-        S.lab[i] = fabs(S.d[S.ord[i]]);
-        S.ord2[i] = i;
-      }
-      for (int i = 0; i < b; ++i)
-        for (int j = i + 1; j < b; ++j)
-          if (S.lab[S.ord2[i]] > S.lab[S.ord2[j]]) {
-            const int t = S.ord2[i];
-            S.ord2[i] = S.ord2[j];
-            S.ord2[j] = t;
-          }
-    }
+    he_order(S.d, S.ord, b, &S.tie);
+    for (int i = tid; i < b; i += nth) S.lab[i] = fabs(S.d[S.ord[i]]);
     __syncthreads();
+    he_order(S.lab, S.ord2, b, &S.tie);
     for (int i = tid; i < b; i += nth) a.w2_all[((size_t)pt * a.ndisp + dsp) * b + i] = S.lab[i];
     if (vecs) {
       // ---------------------------------------- back-transformation V = Q D Z
@@ -416,18 +488,29 @@ __global__ void __launch_bounds__(kHeThreads) heev_kernel(PhononArgs a, int nmat
         __syncthreads();
         for (int j = tid; j < b; j += nth) {
           double2 s = make_double2(0.0, 0.0);
+          double2* Vj = V + (size_t)(k + 1) * b + j;
+#pragma unroll 8
           for (int i = 0; i < m; ++i) {  // v^H y
-            const double2 v = S.v[i], y = V[(size_t)(k + 1 + i) * b + j];
+            const double2 v = S.v[i], y = Vj[(size_t)i * b];
             s.x += v.x * y.x + v.y * y.y;
             s.y += v.x * y.y - v.y * y.x;
           }
           s.x *= tau;
           s.y *= tau;
-          for (int i = 0; i < m; ++i) {
-            const double2 t = cmul(S.v[i], s);
-            double2* y = V + (size_t)(k + 1 + i) * b + j;
-            const double2 o = *y;
-            *y = make_double2(o.x - t.x, o.y - t.y);
+          int i = 0;
+          for (; i + 8 <= m; i += 8) {  // eight rows loaded before the first is stored
+            double2 o[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) o[r] = Vj[(size_t)(i + r) * b];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+              const double2 t = cmul(S.v[i + r], s);
+              Vj[(size_t)(i + r) * b] = make_double2(o[r].x - t.x, o[r].y - t.y);
+            }
+          }
+          for (; i < m; ++i) {
+            const double2 t = cmul(S.v[i], s), o = Vj[(size_t)i * b];
+            Vj[(size_t)i * b] = make_double2(o.x - t.x, o.y - t.y);
           }
         }
         __syncthreads();
@@ -463,7 +546,11 @@ cudaError_t launch_heev(const PhononArgs& a, cudaStream_t s) {
   const int b = a.geo.b;
   if (b < 1 || b > kHeMaxB || !a.he_work) return cudaErrorInvalidValue;
   const int nmat = a.geo.nkc * a.ndisp;
-  heev_kernel<<<std::min(heev_slots(nmat), a.he_slots), kHeThreads, 0, s>>>(a, nmat);
+  const int grid = std::min(heev_slots(nmat), a.he_slots);
+  // more matrices than two CTAs per SM take at once: four per SM (448 matrices
+  // of 192 bands: 32.1 ms against 37.1; 224 of 84 bands: 4.8 against 4.1)
+  if (grid > 2 * 148) heev_kernel<4><<<grid, kHeThreads, 0, s>>>(a, nmat);
+  else heev_kernel<2><<<grid, kHeThreads, 0, s>>>(a, nmat);
   return cudaGetLastError();
 }
 
