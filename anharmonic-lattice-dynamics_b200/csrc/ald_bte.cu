@@ -393,7 +393,21 @@ struct CgDev {
 // loads serves all the rows, and small matrices still give n/kGemvRows
 // blocks.  With vec (rows 16-byte aligned) A is read as 16-byte vectors,
 // else element-wise.  The products are summed in double.
-constexpr int kGemvRows = 4;
+//
+// Bound by the one read of A.  The kernels of an iteration are launched as
+// programmatic dependents: while the vector kernels before it run (a tenth of
+// an iteration at n = 16000), the blocks of the first wave are resident and
+// bring the start of their rows into L2; nothing else is touched before the
+// wait.  The warps interleave over a row, so those bytes are the first ones
+// read.  FP32 matrices were bound by the conversion to double (one per
+// element, on a unit a quarter as wide as the FP64 one); widen() does it with
+// two shifts, a mask and a product.  Per iteration at n = 16000 FP32: 196 us
+// before, 168 us now; at n = 9000 FP64: 136 and 108 us (the reads alone: 155
+// and 99).  Two rows to a block keep more blocks resident than four: 16.2
+// against 18.0 ms for the 94 iterations in FP32, 9.6 against 10.2 ms for 86 in
+// FP64.
+constexpr int kGemvRows = 2;
+constexpr unsigned kGemvAhead = 16384;  // bytes of each row brought in before the wait
 
 template <class T>
 struct Vec16;
@@ -407,10 +421,22 @@ template <>
 struct Vec16<float> {
   using t = float4;
   static constexpr int w = 4;
-  __device__ static double at(const float4& v, int i) {
-    return (double)(i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w);
-  }
+  __device__ static float at(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 };
+
+// A finite float as a double, exactly, without the conversion unit: the
+// float's exponent and mantissa moved into a double's fields read as
+// x * 2^-896 (zeros and subnormals too), and the product with 2^896 is exact.
+// Infinities and NaNs come out finite; probe (a sum of x * 0) turns NaN then.
+__device__ __forceinline__ double widen(float x, float& probe) {
+  const int i = __float_as_int(x);
+  probe = fmaf(x, 0.f, probe);
+  return __hiloint2double((i >> 3) & (int)0x8fffffffu, i << 29) * 0x1p896;
+}
+__device__ __forceinline__ double widen(double x, float&) { return x; }
+
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class T>
 __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n, size_t ld, int vec,
@@ -418,9 +444,16 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n,
                                                                const double* __restrict__ x, double* __restrict__ y,
                                                                double* partial, const double* g, double* partial_g,
                                                                const CgDev* st) {
-  if (st && st->done) return;
   using V = typename Vec16<T>::t;
   constexpr int W = Vec16<T>::w;
+  pdl_launch();
+  if (st && vec && threadIdx.x < kGemvRows) {
+    const T* a = A + (size_t)min((int)(blockIdx.x * kGemvRows + threadIdx.x), nrows - 1) * ld;
+    const unsigned bytes = min((size_t)kGemvAhead, (size_t)(n / W) * 16);
+    if (bytes) asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(bytes) : "memory");
+  }
+  pdl_wait();
+  if (st && st->done) return;
   __shared__ double red[kGemvWarps][kGemvRows];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row0 = blockIdx.x * kGemvRows;
@@ -430,13 +463,12 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n,
   double acc[kGemvRows];
 #pragma unroll
   for (int r = 0; r < kGemvRows; ++r) acc[r] = 0.0;
-  // this warp's slice of the vectors [v0, v1), then of the scalar tail
+  // the vectors, then the scalar tail
   const int nv = vec ? n / W : 0;
-  const int per = (nv + kGemvWarps - 1) / kGemvWarps;
-  const int v0 = warp * per, v1 = min(nv, v0 + per);
+  float probe = 0.f;
   const double2* x2 = reinterpret_cast<const double2*>(x);
-#pragma unroll 2
-  for (int v = v0 + lane; v < v1; v += 32) {
+#pragma unroll sizeof(T) == 8 ? 4 : 2
+  for (int v = threadIdx.x; v < nv; v += 32 * kGemvWarps) {
     double xv[W];
 #pragma unroll
     for (int h = 0; h < W / 2; ++h) {
@@ -446,11 +478,20 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n,
     }
     V av[kGemvRows];
 #pragma unroll
-    for (int r = 0; r < kGemvRows; ++r) av[r] = __ldg(reinterpret_cast<const V*>(Ar[r]) + v);
+    for (int r = 0; r < kGemvRows; ++r) av[r] = __ldcs(reinterpret_cast<const V*>(Ar[r]) + v);
 #pragma unroll
     for (int r = 0; r < kGemvRows; ++r)
 #pragma unroll
-      for (int i = 0; i < W; ++i) acc[r] = fma(Vec16<T>::at(av[r], i), xv[i], acc[r]);
+      for (int i = 0; i < W; ++i) acc[r] = fma(widen(Vec16<T>::at(av[r], i), probe), xv[i], acc[r]);
+  }
+  if (probe != probe) {  // an infinity or a NaN in these rows: the conversion that knows them
+#pragma unroll
+    for (int r = 0; r < kGemvRows; ++r) {
+      acc[r] = 0.0;
+      for (int v = threadIdx.x; v < nv; v += 32 * kGemvWarps)
+        for (int i = 0; i < W; ++i)
+          acc[r] = fma((double)Ar[r][(size_t)v * W + i], x[(size_t)v * W + i], acc[r]);
+    }
   }
   for (int j = nv * W + warp * 32 + lane; j < n; j += 32 * kGemvWarps) {
     const double xj = x[j];
@@ -519,20 +560,42 @@ __global__ void cg_init_kernel(int n, const double* y, const double* b, double* 
 constexpr int kCgThreads = 256;
 constexpr int kCgBlocksMax = 64;
 
+// N sums over the block at once (one exchange), the results in every thread
+template <int N>
+__device__ __forceinline__ void cg_block_sums(double (&v)[N]) {
+  __shared__ double red[kCgThreads / 32][N];
+#pragma unroll
+  for (int k = 0; k < N; ++k)
+    for (int o = 16; o > 0; o >>= 1) v[k] += __shfl_xor_sync(0xffffffffu, v[k], o);
+  if ((threadIdx.x & 31) == 0)
+#pragma unroll
+    for (int k = 0; k < N; ++k) red[threadIdx.x >> 5][k] = v[k];
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; ++k) {
+    v[k] = red[0][k];
+#pragma unroll
+    for (int w = 1; w < kCgThreads / 32; ++w) v[k] += red[w][k];
+  }
+}
+
 // alpha = (grad . conj) / (conj . A conj); x -= alpha conj; grad -= alpha aux;
 // per-CTA partial sums of x.x, conj.conj, grad_new.grad_new, grad_old.grad_old
 __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(int n, const double* aux, const double* pden,
                                                               const double* pnum, int nparts, double* grad,
                                                               const double* conj, double* v0, double* x,
                                                               double* p4, CgDev* st) {
+  pdl_launch();
+  pdl_wait();
   if (st->done) return;
-  double num = 0, den = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
-    num += pnum[i];
-    den += pden[i];
+  double nd[2] = {0, 0};
+#pragma unroll 8
+  for (int i = threadIdx.x; i < nparts; i += kCgThreads) {
+    nd[0] += pnum[i];
+    nd[1] += pden[i];
   }
-  num = vblock_sum(num);
-  den = vblock_sum(den);
+  cg_block_sums<2>(nd);
+  const double num = nd[0], den = nd[1];
   const double alpha = num / den;
   double v2 = 0, cc = 0, gg = 0, g2 = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -548,15 +611,11 @@ __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(int n, const doub
     gg += gn * gn;
     g2 += gi * gi;
   }
-  v2 = vblock_sum(v2);
-  cc = vblock_sum(cc);
-  gg = vblock_sum(gg);
-  g2 = vblock_sum(g2);
+  double q[4] = {v2, cc, gg, g2};
+  cg_block_sums<4>(q);
   if (threadIdx.x == 0) {
-    p4[0 * kCgBlocksMax + blockIdx.x] = v2;
-    p4[1 * kCgBlocksMax + blockIdx.x] = cc;
-    p4[2 * kCgBlocksMax + blockIdx.x] = gg;
-    p4[3 * kCgBlocksMax + blockIdx.x] = g2;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p4[k * kCgBlocksMax + blockIdx.x] = q[k];
     if (blockIdx.x == 0) {
       st->num = num;
       st->den = den;
@@ -567,12 +626,18 @@ __global__ void __launch_bounds__(kCgThreads) cg_update_kernel(int n, const doub
 // the stop rule; unless it fires, conj = -grad + beta conj with beta = gg/g2
 __global__ void __launch_bounds__(kCgThreads) cg_dir_kernel(int n, const double* p4, const double* grad,
                                                            double* conj, CgDev* st, int mode, double tol) {
+  pdl_launch();
+  pdl_wait();
   if (st->done) return;
   __shared__ double s4[4];
-  if (threadIdx.x < 4) {
+  const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (wp < 4) {  // kCgBlocksMax = 64 partials: two per lane
     double t = 0;
-    for (int k = 0; k < (int)gridDim.x; ++k) t += p4[threadIdx.x * kCgBlocksMax + k];
-    s4[threadIdx.x] = t;
+#pragma unroll
+    for (int h = 0; h < kCgBlocksMax; h += 32)
+      if (h + lane < (int)gridDim.x) t += p4[wp * kCgBlocksMax + h + lane];
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (lane == 0) s4[wp] = t;
   }
   __syncthreads();
   const double v2 = s4[0], cc = s4[1], gg = s4[2], g2 = s4[3];
@@ -725,14 +790,28 @@ static cudaError_t capture_cg(int iters, int n, size_t ld, int vec, int nblk, co
   std::lock_guard<std::mutex> cap(capture_mutex());
   cudaError_t e = cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return e;
-  for (int it = 0; it < iters; ++it) {
-    gemv_kernel<T><<<nblk, kGemvWarps * 32, 0, s>>>(n, n, ld, vec, dA, w.conj.p, w.aux.p, w.partial.p, w.grad.p,
-                                                     w.pnum.p, st);
-    cg_update_kernel<<<nb, kCgThreads, 0, s>>>(n, w.aux.p, w.partial.p, w.pnum.p, nblk, w.grad.p, w.conj.p, w.v0.p,
-                                               dx, w.p4.p, st);
-    cg_dir_kernel<<<nb, kCgThreads, 0, s>>>(n, w.p4.p, w.grad.p, w.conj.p, st, mode, tol);
+  cudaLaunchAttribute pdl{};
+  pdl.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  pdl.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t g{}, v{};
+  g.gridDim = nblk;
+  g.blockDim = kGemvWarps * 32;
+  v.gridDim = nb;
+  v.blockDim = kCgThreads;
+  g.stream = v.stream = s;
+  g.attrs = v.attrs = &pdl;
+  v.numAttrs = 1;
+  const double *conj = w.conj.p, *grad = w.grad.p, *aux = w.aux.p, *den = w.partial.p, *num = w.pnum.p, *p4 = w.p4.p;
+  const CgDev* stc = st;
+  for (int it = 0; it < iters && e == cudaSuccess; ++it) {
+    g.numAttrs = it > 0;  // the first follows whatever ran before the graph
+    e = cudaLaunchKernelEx(&g, gemv_kernel<T>, n, n, ld, vec, dA, conj, w.aux.p, w.partial.p, grad, w.pnum.p, stc);
+    if (e == cudaSuccess)
+      e = cudaLaunchKernelEx(&v, cg_update_kernel, n, aux, den, num, nblk, w.grad.p, conj, w.v0.p, dx, w.p4.p, st);
+    if (e == cudaSuccess) e = cudaLaunchKernelEx(&v, cg_dir_kernel, n, p4, grad, w.conj.p, st, mode, tol);
   }
-  e = cudaStreamEndCapture(s, &graph);
+  const cudaError_t ended = cudaStreamEndCapture(s, &graph);
+  if (e == cudaSuccess) e = ended;
   if (e == cudaSuccess) e = cudaGraphInstantiate(out, graph, 0);
   if (graph) cudaGraphDestroy(graph);
   return e;
@@ -750,8 +829,7 @@ static int cg_device_t(int n, size_t ld, const T* dA, const double* db, double* 
   const int vec = ((uintptr_t)dA & 15u) == 0 && (ld * sizeof(T)) % 16 == 0;  // rows 16-byte aligned
   if (w.grad.alloc(n) || w.conj.alloc(n) || w.aux.alloc(n) || w.v0.alloc(n) || w.partial.alloc(nblk) ||
       w.pnum.alloc(nblk) || w.p4.alloc(4 * kCgBlocksMax) ||
-      w.fmin.alloc(1) || w.st.alloc(sizeof(CgDev)) ||
-      (!w.h_done && cudaHostAlloc((void**)&w.h_done, sizeof(int), cudaHostAllocDefault) != cudaSuccess)) {
+      w.fmin.alloc(1) || w.st.alloc(sizeof(CgDev))) {
     msg = "cg: allocation failed";
     return ALD_ERR_NOMEM;
   }
@@ -787,9 +865,10 @@ static int cg_device_t(int n, size_t ld, const T* dA, const double* db, double* 
     e = cudaGraphLaunch(full ? w.exec : w.exec_tail, s);
     done += full ? chunk : tail;
     if (e == cudaSuccess && done < max_iter) {
-      e = cudaMemcpyAsync(w.h_done, &st->done, sizeof(int), cudaMemcpyDeviceToHost, s);
+      int stop = 0;  // not pinned: pinning a page takes 1.5 to 20 ms of a context's first solve
+      e = cudaMemcpyAsync(&stop, &st->done, sizeof stop, cudaMemcpyDeviceToHost, s);
       if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-      if (e == cudaSuccess && *w.h_done) break;
+      if (e == cudaSuccess && stop) break;
     }
   }
   if (e != cudaSuccess) {

@@ -559,7 +559,6 @@ struct CgWork {
   DevBuf<char> st;
   cudaGraphExec_t exec = nullptr;       // kCgChunk iterations
   cudaGraphExec_t exec_tail = nullptr;  // max_iter % kCgChunk iterations
-  int* h_done = nullptr;                // pinned copy of the stop flag
   int n = -1, max_iter = -1, mode = -1;
   double tol = 0;
   const void* A = nullptr;
@@ -569,7 +568,6 @@ struct CgWork {
   ~CgWork() {
     if (exec) cudaGraphExecDestroy(exec);
     if (exec_tail) cudaGraphExecDestroy(exec_tail);
-    if (h_done) cudaFreeHost(h_done);
   }
 };
 int cg_device(int n, const double* dA /*row-major*/, const double* db, double* dx, int max_iter, int mode,
