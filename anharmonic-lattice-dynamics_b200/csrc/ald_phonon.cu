@@ -298,8 +298,7 @@ __global__ void __launch_bounds__(kThreads) phonon_kernel(PhononArgs a) {
 }
 
 // ------------------------------------------------------------------
-// Small cells (b <= 12): G matrices per warp (32/G lanes each: G = 4 up to 4
-// bands, 2 up to 8, else 1), kPhWarps warps per CTA, synchronised with
+// Small cells (b <= 12): G matrices per warp (32/G lanes each), kPhWarps warps per CTA, synchronised with
 // __syncwarp only.  Every lane runs the same sequence of __syncwarp and
 // shuffle calls: a matrix that has converged (or a slot past the last
 // matrix) just stops doing work.  The same arithmetic as phonon_kernel
@@ -637,18 +636,27 @@ __global__ void freq_dist_kernel(Geometry geo, const double* w2, double cnst, do
 
 cudaError_t launch_phonons(const PhononArgs& a, cudaStream_t s) {
   int b = a.geo.b;
-  const int G = b <= 4 ? 4 : (b <= 8 ? 2 : 1);  // matrices per warp
-  const size_t smw = (size_t)kPhWarps * G * (2 * (size_t)b * b + a.nuniq) * sizeof(double2);
+  // Matrices per warp: the rotations of a round take few lanes (three of 6
+  // bands'), so packing more matrices saves issue slots once there are enough
+  // warps to cover the latency (109760 matrices of 6 bands: two to a warp 2.09 ms, four
+  // 1.47, eight 1.49; 40 matrices: 74, 99 and 140 us).
+  const int few = b <= 4 ? 4 : (b <= 8 ? 2 : 1);
+  const size_t per = kPhWarps * (2 * (size_t)b * b + a.nuniq) * sizeof(double2);
+  const bool many = b <= 8 && a.geo.nkc * (long long)a.ndisp >= 148LL * 16 * 2 * few && 2 * few * per <= 64 * 1024;
+  const int G = many ? 2 * few : few;
+  const size_t smw = G * per;
   if (b <= kPhBMax && smw <= 160 * 1024) {
     const int nmat = a.geo.nkc * a.ndisp;
     const int per_cta = kPhWarps * G;
     cudaError_t e = cudaSuccess;
 #define ALD_PHW(GG)                                                                                            \
-  if (smw > 48 * 1024)                                                                                         \
+  if (smw > 24 * 1024) /* with the static arrays, up to 24 KB */                                               \
     e = raise_smem_limit((const void*)phonon_warp_kernel<GG>, smw);                                            \
   if (e != cudaSuccess) return e;                                                                              \
   phonon_warp_kernel<GG><<<(nmat + per_cta - 1) / per_cta, kPhWarps * 32, smw, s>>>(a, nmat);
-    if (G == 4) {
+    if (G == 8) {
+      ALD_PHW(8)
+    } else if (G == 4) {
       ALD_PHW(4)
     } else if (G == 2) {
       ALD_PHW(2)
