@@ -280,7 +280,6 @@ struct SelfArgs {
   double* part;              // self_partial_doubles(*this)
   int* err;
 };
-size_t self_smem_bytes(const SelfArgs& a, int* ppb);
 size_t self_partial_doubles(const SelfArgs& a);
 cudaError_t launch_k3_points(int np, int nkc, const double* qp, const double* kpc, double* k3, cudaStream_t s);
 // out: np*b*4 = nself re, im, uself re, im per (p, la), already /nkc*pi
