@@ -392,6 +392,7 @@ struct CgDev {
   double num, den, err;
   int done, iters;
   double bnorm;
+  double fmin;
 };
 
 // y = A x for a row-major A of nrows x n (leading dimension ld) of double or
@@ -697,7 +698,7 @@ __global__ void __launch_bounds__(256) cg_dots_kernel(int n, const double* aux, 
   }
 }
 
-__global__ void cg_fmin_kernel(int n, const double* x, const double* Ax, const double* b, double* out) {
+__global__ void cg_fmin_kernel(int n, const double* x, const double* Ax, const double* b, CgDev* st) {
   double s1 = 0, s2 = 0;
   for (int i = threadIdx.x; i < n; i += blockDim.x) {
     s1 += x[i] * Ax[i];
@@ -705,7 +706,7 @@ __global__ void cg_fmin_kernel(int n, const double* x, const double* Ax, const d
   }
   s1 = vblock_sum(s1);
   s2 = vblock_sum(s2);
-  if (threadIdx.x == 0) *out = 0.5 * s1 - s2;
+  if (threadIdx.x == 0) st->fmin = 0.5 * s1 - s2;
 }
 
 }  // namespace
@@ -838,7 +839,7 @@ static int cg_device_t(int n, size_t ld, const T* dA, const double* db, double* 
   const int vec = ((uintptr_t)dA & 15u) == 0 && (ld * sizeof(T)) % 16 == 0;  // rows 16-byte aligned
   if (w.grad.alloc(n) || w.conj.alloc(n) || w.aux.alloc(n) || w.v0.alloc(n) || w.partial.alloc(nblk) ||
       w.pnum.alloc(nblk) || w.p4.alloc(4 * kCgBlocksMax) ||
-      w.fmin.alloc(1) || w.st.alloc(sizeof(CgDev))) {
+      w.st.alloc(sizeof(CgDev))) {
     msg = "cg: allocation failed";
     return ALD_ERR_NOMEM;
   }
@@ -886,16 +887,16 @@ static int cg_device_t(int n, size_t ld, const T* dA, const double* db, double* 
   }
   gemv_kernel<T><<<nblk, kGemvWarps * 32, 0, s>>>(n, n, ld, vec, dA, dx, w.aux.p, nullptr, nullptr, nullptr,
                                                    nullptr);
-  cg_fmin_kernel<<<1, kVecThreads, 0, s>>>(n, dx, w.aux.p, db, w.fmin.p);
+  cg_fmin_kernel<<<1, kVecThreads, 0, s>>>(n, dx, w.aux.p, db, st);
   CgDev h;
   e = cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(funcmin, w.fmin.p, sizeof(double), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     msg = std::string("cg: ") + cudaGetErrorString(e);
     return ALD_ERR_CUDA;
   }
   *iters = h.iters;
+  *funcmin = h.fmin;
   *err_out = h.err;
   return h.done ? ALD_OK : ALD_WARN_CG_MAXITER;
 }
@@ -918,7 +919,7 @@ static int cg_rows_t(int n, int row0, int nrows, size_t ld, const T* dA, const d
   const int nblk = (nrows + kGemvRows - 1) / kGemvRows;
   const int nb = std::min(kCgBlocksMax, (n + kCgThreads - 1) / kCgThreads);
   if (w.grad.alloc(n) || w.conj.alloc(n) || w.aux.alloc(n) || w.v0.alloc(n) || w.partial.alloc(nb) ||
-      w.pnum.alloc(nb) || w.p4.alloc(4 * kCgBlocksMax) || w.fmin.alloc(1) || w.st.alloc(sizeof(CgDev)) ||
+      w.pnum.alloc(nb) || w.p4.alloc(4 * kCgBlocksMax) || w.st.alloc(sizeof(CgDev)) ||
       w.yloc.alloc(std::max(nrows, 1))) {
     msg = "cg: allocation failed";
     return ALD_ERR_NOMEM;
@@ -962,15 +963,15 @@ static int cg_rows_t(int n, int row0, int nrows, size_t ld, const T* dA, const d
     msg = "cg: the exchange of A x failed";
     return r;
   }
-  cg_fmin_kernel<<<1, kVecThreads, 0, s>>>(n, dx, w.aux.p, db, w.fmin.p);
+  cg_fmin_kernel<<<1, kVecThreads, 0, s>>>(n, dx, w.aux.p, db, st);
   cudaError_t e = cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(funcmin, w.fmin.p, sizeof(double), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   if (e != cudaSuccess) {
     msg = std::string("cg: ") + cudaGetErrorString(e);
     return ALD_ERR_CUDA;
   }
   *iters = h.iters;
+  *funcmin = h.fmin;
   *err_out = h.err;
   return h.done ? ALD_OK : ALD_WARN_CG_MAXITER;
 }

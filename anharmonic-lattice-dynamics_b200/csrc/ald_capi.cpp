@@ -202,6 +202,10 @@ int check_err_flags(ald_ctx* c) {
   int h = 0;
   CK(cudaMemcpyAsync(&h, c->err.p, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
   CK(cudaStreamSynchronize(c->stream));
+  return act_on_err_flags(c, h);
+}
+
+int act_on_err_flags(ald_ctx* c, int h) {
   if (h) {
     CK(cudaMemsetAsync(c->err.p, 0, sizeof(int), c->stream));
     if (h & 64) c->det_overflow = true;  // no error: the pipeline runs again with the two-pass delta

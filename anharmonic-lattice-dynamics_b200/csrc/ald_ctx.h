@@ -2,10 +2,34 @@
 // translation units (ald_capi.cpp, ald_pipeline.cpp).
 #pragma once
 #include <string>
+#include <vector>
 
 #include "ald_internal.h"
 
 using namespace ald;
+
+// timing events of a pipeline call, kept for the next one
+struct EventPool {
+  std::vector<cudaEvent_t> ev;
+  size_t used = 0;
+  cudaError_t take(cudaEvent_t* e) {
+    if (used == ev.size()) {
+      const cudaError_t r = cudaEventCreate(e);
+      if (r != cudaSuccess) return r;
+      ev.push_back(*e);
+    } else {
+      *e = ev[used];
+    }
+    ++used;
+    return cudaSuccess;
+  }
+  EventPool() = default;
+  EventPool(const EventPool&) = delete;
+  EventPool& operator=(const EventPool&) = delete;
+  ~EventPool() {
+    for (cudaEvent_t e : ev) cudaEventDestroy(e);
+  }
+};
 
 struct ald_ctx {
   System S;
@@ -42,7 +66,9 @@ struct ald_ctx {
   // phonons and occupations
   DevBuf<double> w2_all, w2, evec, vel, freq, dist, occt;
   // pipeline workspaces, kept across calls (allocation outside the timed work)
-  DevBuf<double> w_R1, w_R2, w_Q, w_v3, w_F, w_x, w_rhs, w_kr, w_kc, w_cm;
+  DevBuf<double> w_R1, w_R2, w_v3, w_F, w_rhs, w_cm;
+  DevBuf<double> w_out, w_Q, w_x, w_kr, w_kc;  // results: one block and its parts
+  EventPool events;
   DevBuf<double> w_R1p, w_R2p, w_Ff, w_Frta, w_part;  // iterative solution: band marginals, F on the mesh
   // isotope scattering (iso=1): g per primitive atom, Piso [ibz][l1] and its partial sums
   std::vector<double> giso;
@@ -77,6 +103,7 @@ namespace ald {
 namespace capi {
 int fail(int code, const std::string& msg);
 int check_err_flags(ald_ctx* c);
+int act_on_err_flags(ald_ctx* c, int flags);  // of flags already read
 int ensure_phonons(ald_ctx* c);
 int ensure_dist(ald_ctx* c, double tempk);
 V3Args v3_args(ald_ctx* c, int first, int nrows, double* out);

@@ -352,7 +352,6 @@ cudaError_t launch_v3_pair_lines(const V3Args& a, const V3LineTables& t, void* w
 cudaError_t launch_v3_lines(const V3Args& a, const V3LineTables& t, void* lines, int precision, cudaStream_t s);
 bool v3_lines_supported(const Geometry& g, const V3LineTables& t);
 // row stage alone, H in FP32 or FP64
-cudaError_t launch_v3_rows_f32(const V3Args& a, cudaStream_t s);
 cudaError_t launch_v3_rows_f64(const V3Args& a, cudaStream_t s);
 // more than 12 bands (ald_v3_dense.cu): the class sums and both mode products
 // as batched complex GEMMs per (q1, q2) pair; hbuf from launch_v3_rows_f64;
@@ -553,7 +552,7 @@ cudaError_t launch_update(const Geometry& geo, int n1_first, int nrows, const in
 // iteration loop, kept across calls and re-captured only when the problem
 // (size, pointers, stop rule) changes
 struct CgWork {
-  DevBuf<double> grad, conj, aux, v0, partial, pnum, p4, fmin;
+  DevBuf<double> grad, conj, aux, v0, partial, pnum, p4;
   DevBuf<double> yloc;  // the local rows of A v (row-sharded CG)
   DevBuf<char> st;
   cudaGraphExec_t exec = nullptr;       // kCgChunk iterations

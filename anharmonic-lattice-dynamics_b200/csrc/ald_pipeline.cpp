@@ -34,12 +34,13 @@ namespace {
 
 struct StageTimer {
   cudaStream_t s;
+  EventPool* pool;  // the context's events, reused from call to call
   std::vector<std::pair<int, std::pair<cudaEvent_t, cudaEvent_t>>> marks;
   cudaEvent_t open_ev = nullptr;
   int open_stage = -1;
   cudaError_t begin(int stage) {
     cudaEvent_t e;
-    cudaError_t r = cudaEventCreate(&e);
+    cudaError_t r = pool->take(&e);
     if (r != cudaSuccess) return r;
     open_ev = e;
     open_stage = stage;
@@ -47,7 +48,7 @@ struct StageTimer {
   }
   cudaError_t end() {
     cudaEvent_t e;
-    cudaError_t r = cudaEventCreate(&e);
+    cudaError_t r = pool->take(&e);
     if (r != cudaSuccess) return r;
     r = cudaEventRecord(e, s);
     marks.push_back({open_stage, {open_ev, e}});
@@ -60,13 +61,6 @@ struct StageTimer {
       cudaEventElapsedTime(&t, m.second.first, m.second.second);
       ms[m.first] += t;
     }
-  }
-  ~StageTimer() {
-    for (auto& m : marks) {
-      cudaEventDestroy(m.second.first);
-      cudaEventDestroy(m.second.second);
-    }
-    if (open_ev) cudaEventDestroy(open_ev);
   }
 };
 
@@ -120,17 +114,12 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   cudaStream_t s = c->stream;
   StageTimer tm;
   tm.s = s;
+  tm.pool = &c->events;
+  c->events.used = 0;
   const int b = c->geo.b, nkc = c->T.nkc, nibz = c->T.nibz;
   cudaEvent_t t0, t1;
-  ALD_CK(cudaEventCreate(&t0));
-  ALD_CK(cudaEventCreate(&t1));
-  struct EvGuard {
-    cudaEvent_t a, b;
-    ~EvGuard() {
-      cudaEventDestroy(a);
-      cudaEventDestroy(b);
-    }
-  } evg{t0, t1};
+  ALD_CK(c->events.take(&t0));
+  ALD_CK(c->events.take(&t1));
   ALD_CK(cudaEventRecord(t0, s));
   // ---- 0: phonons and occupations
   ALD_CK(tm.begin(0));
@@ -183,7 +172,13 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
     ALD_CKA(c->w_R1p.alloc(rsz));
     ALD_CKA(c->w_R2p.alloc(rsz));
   }
-  ALD_CKA(Q.alloc((size_t)3 * nibz * b));
+  // what goes back to the host lies in one block, read with one copy at the
+  // end: the error flags, kappa (RTA, CG), Q, the solution
+  const size_t N = (size_t)3 * b * nibz;
+  const size_t o_kr = 32, o_kc = o_kr + 9 * (size_t)b, o_Q = o_kc + 9 * (size_t)b;
+  const size_t o_x = (o_Q + (size_t)3 * nibz * b + 31) / 32 * 32;  // read as vectors
+  ALD_CKA(c->w_out.alloc(o_x + N));
+  Q.view_of(c->w_out.p + o_Q, (size_t)3 * nibz * b);
   const int gauss = delta_mode(c) == ALD_DELTA_GAUSS;
   // tetrahedron: weights straight into R1/R2 (no corner-energy/weight arrays)
   // the delta kernels read |V3|^2 slice by slice (coalesced over q2): the
@@ -359,7 +354,6 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   ALD_CK(tm.end());
   // ---- 4: RTA
   KappaArgs k = kappa_args(c, tempk);
-  const size_t N = (size_t)3 * b * nibz;
   DevBuf<double>& F = c->w_F;
   DevBuf<double>& x = c->w_x;
   DevBuf<double>& rhs = c->w_rhs;
@@ -367,10 +361,10 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   DevBuf<double>& kc = c->w_kc;
   DevBuf<double>& cm = c->w_cm;
   ALD_CKA(F.alloc(N));
-  ALD_CKA(x.alloc(N));
+  x.view_of(c->w_out.p + o_x, N);
   ALD_CKA(rhs.alloc(N));
-  ALD_CKA(kr.alloc((size_t)9 * b));
-  ALD_CKA(kc.alloc((size_t)9 * b));
+  kr.view_of(c->w_out.p + o_kr, (size_t)9 * b);
+  kc.view_of(c->w_out.p + o_kc, (size_t)9 * b);
   ALD_CK(tm.begin(4));
   ALD_CK(launch_rta_F(k, dQ, F.p, s));
   ALD_CK(launch_kappa(k, F.p, 0, kr.p, c->err.p, s));
@@ -509,23 +503,19 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   ALD_CK(tm.end());
   ALD_CK(cudaEventRecord(t1, s));
   // ---- results to the host
-  std::vector<double> hkr((size_t)9 * b), hkc((size_t)9 * b);
-  ALD_CK(cudaMemcpyAsync(hkr.data(), kr.p, hkr.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  ALD_CK(cudaMemcpyAsync(hkc.data(), kc.p, hkc.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-  double d2h = 2.0 * hkr.size() * sizeof(double);
-  std::vector<double> hq;
-  if (Qo || QNo || QUo) {
-    hq.resize((size_t)3 * nibz * b);
-    ALD_CK(cudaMemcpyAsync(hq.data(), Q.p, hq.size() * sizeof(double), cudaMemcpyDeviceToHost, s));
-    d2h += hq.size() * sizeof(double);
-  }
-  if (xo) {
-    ALD_CK(cudaMemcpyAsync(xo, x.p, N * sizeof(double), cudaMemcpyDeviceToHost, s));
-    d2h += N * sizeof(double);
-  }
+  const bool want_q = Qo || QNo || QUo;
+  const size_t nout = xo ? o_x + N : want_q ? o_Q + (size_t)3 * nibz * b : o_Q;
+  std::vector<double> hout(nout);
+  ALD_CK(cudaMemcpyAsync(c->w_out.p, c->err.p, sizeof(int), cudaMemcpyDeviceToDevice, s));
+  ALD_CK(cudaMemcpyAsync(hout.data(), c->w_out.p, nout * sizeof(double), cudaMemcpyDeviceToHost, s));
   ALD_CK(cudaStreamSynchronize(s));
-  r = check_err_flags(c);
+  const double d2h = (18.0 * b + (want_q ? 3.0 * nibz * b : 0.0) + (xo ? (double)N : 0.0)) * sizeof(double);
+  int flags;
+  std::memcpy(&flags, hout.data(), sizeof flags);
+  r = act_on_err_flags(c, flags);
   if (r) return r;
+  const double *hkr = hout.data() + o_kr, *hkc = hout.data() + o_kc, *hq = hout.data() + o_Q;
+  if (xo) std::memcpy(xo, hout.data() + o_x, N * sizeof(double));
   tm.collect(res->stage_ms);
   float total = 0;
   cudaEventElapsedTime(&total, t0, t1);
@@ -540,8 +530,8 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
     res->kappa_rta[e] = sr;
     res->kappa_cg[e] = sc;
   }
-  if (kappa_rta_modes) std::memcpy(kappa_rta_modes, hkr.data(), hkr.size() * sizeof(double));
-  if (kappa_cg_modes) std::memcpy(kappa_cg_modes, hkc.data(), hkc.size() * sizeof(double));
+  if (kappa_rta_modes) std::memcpy(kappa_rta_modes, hkr, 9 * (size_t)b * sizeof(double));
+  if (kappa_cg_modes) std::memcpy(kappa_cg_modes, hkc, 9 * (size_t)b * sizeof(double));
   for (int i = 0; i < nibz; ++i)
     for (int l = 0; l < b; ++l) {
       if (Qo) Qo[i + (size_t)nibz * l] = hq[(size_t)i * b + l];

@@ -351,13 +351,6 @@ cudaError_t launch_pair_t(const V3Args& a, cudaStream_t s) {
 
 }  // namespace
 
-cudaError_t launch_v3_rows_f32(const V3Args& a, cudaStream_t s) {
-  const int n = a.ncls * 9 * a.geo.b;
-  dim3 rg((n + 255) / 256, a.nrows);
-  v3_row_kernel<float2><<<rg, 256, 0, s>>>(a);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_v3_rows_f64(const V3Args& a, cudaStream_t s) {
   const int n = a.ncls * 9 * a.geo.b;
   dim3 rg((n + 255) / 256, a.nrows);
