@@ -637,13 +637,15 @@ __global__ void freq_dist_kernel(Geometry geo, const double* w2, double cnst, do
 cudaError_t launch_phonons(const PhononArgs& a, cudaStream_t s) {
   int b = a.geo.b;
   // Matrices per warp: the rotations of a round take few lanes (three of 6
-  // bands'), so packing more matrices saves issue slots once there are enough
-  // warps to cover the latency (109760 matrices of 6 bands: two to a warp 2.09 ms, four
-  // 1.47, eight 1.49; 40 matrices: 74, 99 and 140 us).
+  // bands'), so for 5 to 8 bands packing four instead of two saves issue slots
+  // once there are enough warps to cover the latency (6 bands, 109760 matrices:
+  // 2.09 against 1.47 ms, eight 1.49; 40 matrices: 74, 99 and 140 us).  Up to 4
+  // bands eight lanes do better than four (3 bands, 189000 matrices: four to a
+  // warp 1.53 ms, eight 1.92).
   const int few = b <= 4 ? 4 : (b <= 8 ? 2 : 1);
   const size_t per = kPhWarps * (2 * (size_t)b * b + a.nuniq) * sizeof(double2);
-  const bool many = b <= 8 && a.geo.nkc * (long long)a.ndisp >= 148LL * 16 * 2 * few && 2 * few * per <= 64 * 1024;
-  const int G = many ? 2 * few : few;
+  const bool many = few == 2 && a.geo.nkc * (long long)a.ndisp >= 148LL * 16 * 4 && 4 * per <= 64 * 1024;
+  const int G = many ? 4 : few;
   const size_t smw = G * per;
   if (b <= kPhBMax && smw <= 160 * 1024) {
     const int nmat = a.geo.nkc * a.ndisp;
@@ -654,9 +656,7 @@ cudaError_t launch_phonons(const PhononArgs& a, cudaStream_t s) {
     e = raise_smem_limit((const void*)phonon_warp_kernel<GG>, smw);                                            \
   if (e != cudaSuccess) return e;                                                                              \
   phonon_warp_kernel<GG><<<(nmat + per_cta - 1) / per_cta, kPhWarps * 32, smw, s>>>(a, nmat);
-    if (G == 8) {
-      ALD_PHW(8)
-    } else if (G == 4) {
+    if (G == 4) {
       ALD_PHW(4)
     } else if (G == 2) {
       ALD_PHW(2)
