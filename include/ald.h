@@ -41,8 +41,9 @@ enum ald_status {
 
 enum ald_delta { ALD_DELTA_TETRA = 0, ALD_DELTA_GAUSS = 1 };
 /* ALD_MIXED: the V3 contraction in reduced precision with FP32 accumulation --
- * from 9 bands up both eigenvector mode products run on the tensor cores
- * (split-FP16 tcgen05 MMAs), 3 and 6 bands in FP32 on the CUDA cores; from 9
+ * FP32 on the CUDA cores for cells whose pairs fit shared memory (36 bands on
+ * the usual ones), split-FP16 tcgen05 MMAs for the eigenvector mode products
+ * of larger ones; from 9
  * bands up the pairs that involve a mode of vanishing frequency are formed
  * again in FP64.  ALD_MIXED_FP32 uses the FP32 CUDA-core form where one
  * exists.  Inside the pipeline the delta weights and the stored collision
