@@ -407,7 +407,9 @@ struct CgDev {
 // programmatic dependents: while the vector kernels before it run (a tenth of
 // an iteration at n = 16000), the blocks of the first wave are resident and
 // bring the start of their rows into L2; nothing else is touched before the
-// wait.  The warps interleave over a row, so those bytes are the first ones
+// wait.  x (and g, st) is written by the kernels it overlaps: only ordinary
+// loads after the wait see it, so it is neither __restrict__ nor read through
+// the read-only path; A is written by none of them.  The warps interleave over a row, so those bytes are the first ones
 // read.  FP32 matrices were bound by the conversion to double (one per
 // element, on a unit a quarter as wide as the FP64 one); widen() does it with
 // two shifts, a mask and a product.  Per iteration at n = 16000 FP32: 196 us
@@ -449,8 +451,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 
 template <class T>
 __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n, size_t ld, int vec,
-                                                               const T* __restrict__ A,
-                                                               const double* __restrict__ x, double* __restrict__ y,
+                                                               const T* __restrict__ A, const double* x, double* y,
                                                                double* partial, const double* g, double* partial_g,
                                                                const CgDev* st) {
   using V = typename Vec16<T>::t;
@@ -481,7 +482,7 @@ __global__ void __launch_bounds__(kGemvWarps * 32) gemv_kernel(int nrows, int n,
     double xv[W];
 #pragma unroll
     for (int h = 0; h < W / 2; ++h) {
-      const double2 t2 = __ldg(x2 + (size_t)v * (W / 2) + h);
+      const double2 t2 = x2[(size_t)v * (W / 2) + h];
       xv[2 * h] = t2.x;
       xv[2 * h + 1] = t2.y;
     }
