@@ -78,8 +78,8 @@ struct ald_ctx {
   DevBuf<double> w_brange;  // omega range of every band over the mesh
   DevBuf<char> w_scratch;
   DevBuf<double> w_heev;    // Householder eigensolver workspace (large cells)
-  DevBuf<double> w_rmax;    // deterministic delta: low parts of the sums, or each R entry's largest term (FP64 bits)
-  DevBuf<double> w_dscale;  // deterministic delta: its scales and bounds
+  DevBuf<double> w_rmax;    // deterministic delta: lower parts of the sums, or each R entry's largest term (FP64 bits)
+  DevBuf<short> w_dexp;     // deterministic delta: the exponent of each R entry's scale
   bool det_overflow = false;  // a term was beyond the one-pass form's scale (check_err_flags)
   bool det_two_pass = false;  // take the two-pass form
   // launch shapes chosen by ald_autotune (0 = the built-in choices)

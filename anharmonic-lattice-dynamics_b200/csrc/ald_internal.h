@@ -411,10 +411,12 @@ struct CombineArgs {
   unsigned long long* M2 = nullptr;
   unsigned long long* M1p = nullptr;
   unsigned long long* M2p = nullptr;
-  // the one-pass form (mode 3): M1/M2/M1p/M2p hold the low parts of the sums;
-  // scale: 2^S of (process, row, l1, l2), then of (process, row, l1, l3) with
-  // R1p/R2p; err: a term beyond the scale's headroom sets bit 64
-  const double* det_scale = nullptr;
+  // the one-pass form (mode 3): M1/M2/M1p/M2p hold the middle parts of the sums
+  // and, det_lowest entries further on, the lowest ones; det_exp: S of every entry, [process][row][l2][l1][w], then with R1p/R2p
+  // theirs ([process][row][l3][l1][w]); err: a term beyond the headroom of its
+  // entry's scale, or a frequency that nearly vanishes, sets bit 64
+  short* det_exp = nullptr;
+  size_t det_lowest = 0;
   int* err = nullptr;
   double* P1s;               // optional [row][q][l1][l2][l3] (P1smpi)
   double* P2s;
@@ -440,13 +442,12 @@ cudaError_t launch_combine(const CombineArgs& a, void* scratch, cudaStream_t s);
 bool delta_fused_supported(const Geometry& g);
 cudaError_t launch_delta_fused(const CombineArgs& a, cudaStream_t s, int mode = 0);
 cudaError_t launch_delta_finalize(double* R, const unsigned long long* M, size_t n, int b, cudaStream_t s);
-// mode 3, the same in one pass: launch_delta_scale bounds the terms of every
-// (process, row, l1, l2) from |V3|^2 and the Bose factors and forms
-// a.det_scale (work of delta_scale_doubles doubles, det_scale its first
-// part); mode 3 adds the terms in two integer parts of 2^-S and 2^-(S+52);
+// mode 3, the same in one pass: launch_delta_exp bounds the terms of every
+// entry from |V3|^2 and the Bose factors and writes a.det_exp
+// (delta_exp_count values); mode 3 adds the terms in three integer parts;
 // launch_delta_finalize_wide joins them.  R and M zero on entry.
-size_t delta_scale_doubles(int nrows, int b, bool marginals);
-cudaError_t launch_delta_scale(const CombineArgs& a, double* work, cudaStream_t s);
+size_t delta_exp_count(const Geometry& geo, int nrows, bool marginals);
+cudaError_t launch_delta_exp(const CombineArgs& a, cudaStream_t s);
 cudaError_t launch_delta_finalize_wide(const CombineArgs& a, cudaStream_t s);
 // any number of bands (large cells): the tetrahedron or Gaussian delta into
 // R1/R2 and/or P1s/P2s straight from |V3|^2 of the chunk; for the tetrahedron

@@ -213,8 +213,9 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   if (v3_gauss) K = v3_gauss_rows(c);
   if (!v3_gauss) ALD_CKA(v3.alloc(v3f ? (v3n + 1) / 2 : v3n));
   const size_t rchunk = (size_t)K * nkc * b * b;  // entries of one chunk's R1
-  if (det) ALD_CKA(c->w_rmax.alloc((it ? 4 : 2) * rchunk));
-  if (wide) ALD_CKA(c->w_dscale.alloc(delta_scale_doubles(K, b, it != nullptr)));
+  const size_t rmaxn = (size_t)(it ? 4 : 2) * rchunk;
+  if (det) ALD_CKA(c->w_rmax.alloc((wide ? 2 : 1) * rmaxn));
+  if (wide) ALD_CKA(c->w_dexp.alloc(delta_exp_count(c->geo, K, it != nullptr)));
   if (!fused && !any) ALD_CKA(escratch.alloc(std::max<size_t>(256, combine_scratch_bytes(c->geo, K, gauss))));
   ALD_CKA(c->w_brange.alloc((size_t)2 * b));
   ALD_CK(launch_band_range(c->geo, c->freq.p, c->w_brange.p, s));
@@ -280,7 +281,8 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
       a.M2 = M + rchunk;
       a.M1p = it ? M + 2 * rchunk : nullptr;
       a.M2p = it ? M + 3 * rchunk : nullptr;
-      ALD_CK(cudaMemsetAsync(M, 0, (it ? 4 : 2) * rchunk * sizeof(unsigned long long), s));
+      a.det_lowest = rmaxn;
+      ALD_CK(cudaMemsetAsync(M, 0, (wide ? 2 : 1) * rmaxn * sizeof(unsigned long long), s));
     }
     if (fused || (any && !gauss)) {
       ALD_CK(cudaMemsetAsync(a.R1, 0, rbytes, s));
@@ -291,12 +293,12 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
       r = run_v3_gauss(c, v3_args(c, r0, nr, nullptr), a, &res->launches[2]);
       if (r) return r;
     } else if (wide) {
-      a.det_scale = c->w_dscale.p;
+      a.det_exp = c->w_dexp.p;
       a.err = c->err.p;
-      ALD_CK(launch_delta_scale(a, c->w_dscale.p, s));
+      ALD_CK(launch_delta_exp(a, s));
       ALD_CK(launch_delta_fused(a, s, 3));
       ALD_CK(launch_delta_finalize_wide(a, s));
-      res->launches[2] += it ? 7 : 5;
+      res->launches[2] += it ? 8 : 5;
     } else if (det) {
       const size_t n = (size_t)nr * nkc * b * b;
       ALD_CK(launch_delta_fused(a, s, 1));
@@ -570,8 +572,9 @@ extern "C" int ald_kappa_pipeline(ald_ctx* c, double tempk, ald_kappa_result* re
 // device-memory cache, where the next structure of the same sizes finds them)
 static void release_pipeline_workspaces(ald_ctx* c) {
   c->v3c_epoch = 0;  // the kept |V3|^2 goes with its buffer
-  for (DevBuf<double>* b : {&c->w_R1, &c->w_R2, &c->w_v3, &c->w_cm, &c->w_R1p, &c->w_R2p, &c->w_heev, &c->w_rmax, &c->w_dscale})
+  for (DevBuf<double>* b : {&c->w_R1, &c->w_R2, &c->w_v3, &c->w_cm, &c->w_R1p, &c->w_R2p, &c->w_heev, &c->w_rmax})
     b->free();
+  c->w_dexp.free();
   c->w_h.free();
   c->w_h64.free();
   c->w_v3fix.free();

@@ -477,16 +477,23 @@ __global__ void __launch_bounds__(256) q_from_r_kernel(Geometry g, int n1_first,
 // below 2^63 and each rounding is at most 2^-63 x 24 b of the entry.
 // launch_delta_finalize turns the integers back into doubles.
 //
-// MODE 3 (the deterministic option's usual form) needs no first pass: a term
-// is c |V3|^2 n1 G (2pi)^2/(6 nkc), and delta_bound_kernel takes the largest
-// |V3|^2 G of every (process, row, l1, l2) in one read of |V3|^2.  With that
-// bound and kDetCap for the corner weight c, S is chosen so that all kDetTerms
-// terms of an entry stay below 2^61 in units of 2^-S; a term is added as the
-// integer nearest to it in those units and the remainder in units of
-// 2^-(S+52), 113 bits below the bound in all.  The bound may therefore be
-// 2^50 above an entry's own sum before an FP64 sum would have been more exact.
-// A weight beyond kDetCap (a tetrahedron of energies within 1e-6 cm^-1 around
-// omega1) sets bit 64 of the error flag, and the pipeline takes MODE 1 and 2.
+// MODE 3 (the deterministic option's usual form; MODE 4 with the marginals)
+// needs no first pass: a term
+// is c |V3|^2 n1 G (2pi)^2/(6 nkc) with |V3|^2 and G taken at the entry's own
+// point, and delta_bound_kernel forms the largest |V3|^2 G of every entry over
+// l3 in one read of |V3|^2.  With that bound and kDetCap for the corner weight
+// c, the entry's S is chosen so that all its kDetTerms terms stay below 2^61 in
+// units of 2^-S.  A term is split into the integer nearest to it in those
+// units, the remainder in units of 2^-(S+54), and, for terms below 2^-S, what
+// remains of that in units of 2^-(S+108): its 53 bits are kept whole down to
+// 2^-87 of the bound at c = 1, and a smaller one is rounded there.  Between the
+// l3 of an entry |V3|^2 G differs by up to 1/omega3^2 where a frequency nearly
+// vanishes, whether or not that l3 has weight: two parts (2^-33 of the bound)
+// or one S for all points of a (process, row, l1, l2) would then take the other
+// terms' digits.  Below kDetSoft of the largest frequency delta_bound_kernel
+// sets bit 64 of the error flag, as a weight beyond kDetCap does (a tetrahedron
+// of energies within 1e-6 cm^-1 around omega1), and the pipeline takes MODE 1
+// and 2.
 // Rock-salt 16^3 FP64: 14.3 ms in two passes, 8.1 in one (B200; with the
 // queue's two ends, below).
 // corners of make_kp_reg_tet's six tetrahedra (c = o0 + 2 o1 + 4 o2), 3 bits
@@ -514,7 +521,8 @@ __device__ __forceinline__ unsigned long long det_fixed(double v, unsigned long 
   return (unsigned long long)llrint(ldexp(v, 62 - det_exponent(m, b)));
 }
 
-constexpr double kDetCap = 4194304.0;  // 2^22, corner weights in 1/cm^-1
+constexpr double kDetCap = 0x1p22;   // corner weights in 1/cm^-1
+constexpr double kDetSoft = 1e-10;  // of the largest frequency
 
 struct FusedShape {
   int R, nbj, NW, maxrec;
@@ -539,13 +547,22 @@ __host__ __device__ inline FusedShape fused_shape(const Geometry& g) {
   return f;
 }
 
-// a term, scaled by 2^S, into the two integer parts of an entry; false when it
-// is beyond what S leaves room for
-__device__ __forceinline__ bool det_add(double t, int b, double* hi, unsigned long long* lo) {
-  if (!(t < 2305843009213693952.0 / kDetTerms(b))) return false;  // 2^61
-  const double h = rint(t);
-  atomicAdd(reinterpret_cast<unsigned long long*>(hi), (unsigned long long)(long long)h);
-  atomicAdd(lo, (unsigned long long)llrint((t - h) * 4503599627370496.0));  // 2^52
+// 2^s, |s| <= kDetMaxExp
+constexpr int kDetMaxExp = 1000;
+__device__ __forceinline__ double det_pow2(int s) { return __hiloint2double((s + 1023) << 20, 0); }
+
+// a term, scaled by 2^S, into two of an entry's three integer parts (lo, the
+// lowest n2 further on; a remainder is at most half a unit, and kDetTerms(16)
+// of them stay below 2^62): from 1/4 up its last bit is 2^-54 or more, below it
+// has no whole units.  False when it is beyond what S leaves room for
+__device__ __forceinline__ bool det_add(double t, int b, double* hi, unsigned long long* lo, size_t n2) {
+  if (!(fabs(t) < 0x1p61 / kDetTerms(b))) return false;
+  const bool low = fabs(t) < 0.25;
+  const double h = rint(t), r = (t - h) * 0x1p54;
+  const long long l = llrint(r);
+  atomicAdd(low ? lo + n2 : reinterpret_cast<unsigned long long*>(hi),
+            (unsigned long long)llrint(low ? (r - (double)l) * 0x1p54 : h));
+  atomicAdd(lo, (unsigned long long)l);
   return true;
 }
 
@@ -553,7 +570,6 @@ template <int B, bool F32W, class VT, int MODE>
 __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT* __restrict__ v3sq) {
   extern __shared__ __align__(16) unsigned char smraw[];
   __shared__ double s_om[B], s_nb1[B];
-  __shared__ double s_sc[MODE == 3 ? B : 1], s_scp[MODE == 3 ? B : 1];  // 2^S of R, R' per l1
   __shared__ int s_nrec, s_nm, s_ne;  // records; queue entries from the front (mid) and from the back
   __shared__ unsigned short s_lp[kFusedThreads][8];              // window point of each cell corner
   __shared__ unsigned char s_hit[kFusedThreads / 32][32];      // the warp's cells that passed, by lane
@@ -583,7 +599,6 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
   if (tid < b) {
     s_om[tid] = a.freq[(size_t)q1 * b + tid];
     s_nb1[tid] = a.dist[(size_t)q1 * b + tid];
-    if constexpr (MODE == 3) s_sc[tid] = a.det_scale[(((size_t)proc * a.nrows + row) * b + tid) * b + l2];
   }
   // conservative FP32 bounds of omega1 for the range tests (unused bands never count)
   float omlo[B], omhi[B];
@@ -612,7 +627,7 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
   // (2pi)^2/nkc and the 1/6 of the corner weights in one factor
   const double fnorm6 = (2 * PhysConst::pi) * (2 * PhysConst::pi) / nkc / 6.0;
   double* Rp = proc == 0 ? a.R1 : a.R2;
-  double* Rpp = proc == 0 ? a.R1p : a.R2p;  // band marginal over l2 (optional)
+  double* Rpp = MODE == 3 ? nullptr : proc == 0 ? a.R1p : a.R2p;  // band marginal over l2 (optional)
   unsigned long long* Mp = proc == 0 ? a.M1 : a.M2;  // largest terms (MODE 1, 2)
   unsigned long long* Mpp = proc == 0 ? a.M1p : a.M2p;
   // |V3|^2 strides of (q, l1, l2, l3) in the chunk's layout
@@ -664,9 +679,6 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
     if (!((live >> l3) & 1u)) continue;
     __syncthreads();  // window staged / previous slice done
     if (tid == 0) s_nrec = s_nm = s_ne = 0;
-    if constexpr (MODE == 3)
-      if (Rpp && tid < b)
-        s_scp[tid] = a.det_scale[((((size_t)2 + proc) * a.nrows + row) * b + tid) * b + l3];
     for (int p = tid; p < NW; p += blockDim.x) {
       const double fw = s_fw[p], f3 = a.occt[(size_t)l3 * nkc + s_q3[p]];
       s_E[p] = (float)(proc == 0 ? -fw + f3 : fw + f3);
@@ -859,6 +871,9 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
       const double nb1 = s_nb1[l1];
       const size_t o = (size_t)row * nkc * b * b + l1 * b + l2, op = (size_t)row * nkc * b * b + l1 * b + l3;
       const VT* vs = v3row + l2 * s2 + l3 * s3 + l1 * s1;
+      // S of the entries (w, l1, l2), (w, l1, l3)
+      const short* ex = MODE >= 3 ? a.det_exp + ((((size_t)proc * a.nrows + row) * b + l2) * b + l1) * nkc : nullptr;
+      const short* exq = MODE == 4 ? a.det_exp + (((((size_t)2 + proc) * a.nrows + row) * b + l3) * b + l1) * nkc : nullptr;
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const int p = pos_pt[k];
@@ -873,9 +888,9 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
           const unsigned long long bits = (unsigned long long)__double_as_longlong(val);
           atomicMax(Mp + o + w, bits);
           if (Rpp) atomicMax(Mpp + op + w, bits);
-        } else if constexpr (MODE == 3) {
-          if (!det_add(val * s_sc[l1], b, Rp + o + w, Mp + o + w) ||
-              (Rpp && !det_add(val * s_scp[l1], b, Rpp + op + w, Mpp + op + w)))
+        } else if constexpr (MODE >= 3) {
+          if (!det_add(val * det_pow2(__ldg(ex + s_w[p])), b, Rp + o + w, Mp + o + w, a.det_lowest) ||
+              (MODE == 4 && !det_add(val * det_pow2(__ldg(exq + s_w[p])), b, Rpp + op + w, Mpp + op + w, a.det_lowest)))
             atomicOr(a.err, 64);
         } else {
           atomicAdd(reinterpret_cast<unsigned long long*>(Rp + o + w), det_fixed(val, Mp[o + w], b));
@@ -908,88 +923,86 @@ __global__ void delta_finalize_kernel(double* R, const unsigned long long* __res
   }
 }
 
-// A bound of |V3|^2 G for every (process, row, l1, l2) -- and (process, row,
-// l1, l3) for the marginals -- as FP64 bits, at most 2^-20 above the largest
-// (a maximum does not depend on the order).  A CTA takes one slice (l2, l3) of one row; every
-// |V3|^2(q) serves process 1 at w = q and process 2 at w = -q.  One read of
-// |V3|^2, coalesced over q in the slice-major layout.
-template <int B, class VT>
-__global__ void __launch_bounds__(256) delta_bound_kernel(CombineArgs a, const VT* __restrict__ v3sq,
-                                                          unsigned long long* bnd) {
+// S of every entry of MODE 3 and 4 (a.det_exp, [process][row][l2][l1][w]; with
+// MARGINAL those of R', [2 + process][row][l3][l1][w]): kDetTerms terms of at
+// most kDetCap n1 (2pi)^2/(6 nkc) times the largest |V3|^2 G over l3 (l2) stay
+// below 2^61.  A maximum does not depend on the order.  A mode of the running
+// band below kDetSoft, unless the delta zeroes it, sets bit 64.  A thread takes a mesh
+// point q, whose |V3|^2 serves process 1 at w = q and process 2 at w = -q, and
+// a CTA 256 points of one row and l2 (l3).  One read of |V3|^2, coalesced over
+// q in the slice-major layout.
+template <int B, bool MARGINAL, class VT>
+__global__ void __launch_bounds__(256) delta_bound_kernel(CombineArgs a, const VT* __restrict__ v3sq, int lf0) {
   const Geometry& g = a.geo;
-  const int b = g.b, nkc = g.nkc, b2 = b * b, row = blockIdx.y;
-  const int l2 = blockIdx.x / b, l3 = blockIdx.x % b;
+  const int b = g.b, nkc = g.nkc, b2 = b * b, lf = lf0 + blockIdx.y, row = blockIdx.z;
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nkc) return;
   const int q1 = a.mapinv[a.n1_first + row];
-  int m1[3];
+  int m1[3], mq[3], m3[3], mn[3], ins;
   decompose(g, q1, m1);
+  decompose(g, q, mq);
+  const int q3 = pm_index_m(g, m1, mq, 1, ins, m3);
+  for (int x = 0; x < 3; ++x) mn[x] = wrap2(-mq[x], g.nc[x]);
+  const int wn = compose(g, mn);
+  const bool gq = at_gamma_index(g, mq), gn = at_gamma_index(g, mn), g3 = at_gamma_index(g, m3);
   const size_t sq = a.v3_layout == 1 ? 1 : (size_t)b2 * b, s1 = a.v3_layout == 1 ? (size_t)nkc : (size_t)b2;
-  const VT* v = v3sq + (size_t)row * nkc * b2 * b +
-                (a.v3_layout == 1 ? ((size_t)l2 * b + l3) * b * nkc : (size_t)l2 * b + l3);
+  const VT* vr = v3sq + (size_t)row * nkc * b2 * b + (size_t)q * sq;
+  const double* ft = a.occt;
   const double* dt = a.occt + (size_t)nkc * b;
+  double soft = 0.0;
+  for (int l = 0; l < b; ++l) soft = fmax(soft, kDetSoft * a.brange[b + l]);
   // the high words of nonnegative doubles order as the doubles do; one more
   // than the largest, with a zero low word, bounds them all
   int mx1[B], mx2[B];
 #pragma unroll
   for (int l = 0; l < B; ++l) mx1[l] = mx2[l] = 0;
-#pragma unroll 2
-  for (int q = threadIdx.x; q < nkc; q += blockDim.x) {
-    int mq[3], m3[3], mn[3], ins;
-    decompose(g, q, mq);
-    const int q3 = pm_index_m(g, m1, mq, 1, ins, m3);
-    for (int x = 0; x < 3; ++x) mn[x] = wrap2(-mq[x], g.nc[x]);
-    const int wn = compose(g, mn);
-    const double n3 = l3 < 3 && at_gamma_index(g, m3) ? 0.0 : dt[(size_t)l3 * nkc + q3] + 1;
-    const double g1 = l2 < 3 && at_gamma_index(g, mq) ? 0.0 : dt[(size_t)l2 * nkc + q] * n3;
-    const double g2 = l2 < 3 && at_gamma_index(g, mn) ? 0.0 : (dt[(size_t)l2 * nkc + wn] + 1) * n3;
+  for (int lv = 0; lv < b; ++lv) {
+    const int l2 = MARGINAL ? lv : lf, l3 = MARGINAL ? lf : lv;
+    const VT* v = vr + (a.v3_layout == 1 ? ((size_t)l2 * b + l3) * b * nkc : (size_t)l2 * b + l3);
+    const double n3 = l3 < 3 && g3 ? 0.0 : dt[(size_t)l3 * nkc + q3] + 1;
+    const double f1 = l2 < 3 && gq ? 0.0 : dt[(size_t)l2 * nkc + q] * n3;
+    const double f2 = l2 < 3 && gn ? 0.0 : (dt[(size_t)l2 * nkc + wn] + 1) * n3;
+    if (MARGINAL ? !(ft[(size_t)l2 * nkc + q] >= soft) && !(l2 < 3 && gq) : !(ft[(size_t)l3 * nkc + q3] >= soft) && n3 != 0.0)
+      atomicOr(a.err, 64);
 #pragma unroll
     for (int l = 0; l < B; ++l) {
       if (l >= b) continue;
-      const double x = (double)v[(size_t)q * sq + l * s1];
-      mx1[l] = max(mx1[l], __double2hiint(x * g1));
-      mx2[l] = max(mx2[l], __double2hiint(x * g2));
+      const double x = (double)v[l * s1];
+      mx1[l] = max(mx1[l], __double2hiint(x * f1));
+      mx2[l] = max(mx2[l], __double2hiint(x * f2));
     }
   }
-  const size_t nr = (size_t)a.nrows * b2;
+  const double fcap = (2 * PhysConst::pi) * (2 * PhysConst::pi) / nkc / 6.0 * (kDetCap * kDetTerms(b));
+  auto exponent = [&](int hi, double f) {
+    const double x = __hiloint2double(hi + 1, 0) * f;
+    if (!(x < 1.0 / 0.0)) return (short)kDetMaxExp;  // no scale: its terms set the flag
+    int e;
+    frexp(x, &e);
+    return (short)max(-kDetMaxExp, min(kDetMaxExp, 61 - e));
+  };
+  short* e1 = a.det_exp + (((size_t)(MARGINAL ? 2 : 0) * a.nrows + row) * b + lf) * b * nkc;
+  short* e2 = e1 + (size_t)a.nrows * b2 * nkc;
 #pragma unroll
   for (int l = 0; l < B; ++l) {
     if (l >= b) continue;
-    const int h1 = __reduce_max_sync(0xffffffffu, mx1[l]), h2 = __reduce_max_sync(0xffffffffu, mx2[l]);
-    if ((threadIdx.x & 31) == 0) {
-      const unsigned long long x1 = (unsigned long long)(h1 + 1) << 32, x2 = (unsigned long long)(h2 + 1) << 32;
-      const size_t r = ((size_t)row * b + l) * b;
-      atomicMax(bnd + r + l2, x1);
-      atomicMax(bnd + nr + r + l2, x2);
-      if (a.R1p) {
-        atomicMax(bnd + 2 * nr + r + l3, x1);
-        atomicMax(bnd + 3 * nr + r + l3, x2);
-      }
-    }
+    const double f = fcap * a.dist[(size_t)q1 * b + l];
+    e1[(size_t)l * nkc + q] = exponent(mx1[l], f);
+    e2[(size_t)l * nkc + wn] = exponent(mx2[l], f);
   }
 }
 
-// 2^S of every bound: kDetTerms terms of at most bound n1 (2pi)^2/(6 nkc)
-// kDetCap stay below 2^61 (S within +-1000)
-__global__ void delta_scale_kernel(CombineArgs a, const unsigned long long* bnd, double* scale, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const Geometry& g = a.geo;
-  const int b = g.b, l1 = i / b % b, row = i / (b * b) % a.nrows;
-  const double n1 = a.dist[(size_t)a.mapinv[a.n1_first + row] * b + l1];
-  const double fnorm6 = (2 * PhysConst::pi) * (2 * PhysConst::pi) / g.nkc / 6.0;
-  int e;
-  frexp(__longlong_as_double((long long)bnd[i]) * fnorm6 * n1 * (kDetCap * kDetTerms(b)), &e);
-  scale[i] = ldexp(1.0, max(-1000, min(1000, 61 - e)));
-}
-
-// the two integer parts of MODE 3 joined, in place
-__global__ void delta_finalize_wide_kernel(double* R, const unsigned long long* __restrict__ L,
-                                           const double* __restrict__ scale, size_t n, int nkc, int b) {
-  const size_t b2 = (size_t)b * b;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
-    const long long hi = reinterpret_cast<const long long*>(R)[i], lo = (long long)L[i];
-    const size_t row = i / (b2 * nkc);
-    R[i] = ((double)hi + (double)lo * 2.220446049250313e-16) / scale[row * b2 + i % b2];  // 2^-52
-  }
+// the three integer parts of MODE 3 and 4 joined, in place; ex: S of these entries
+__global__ void __launch_bounds__(256) delta_finalize_wide_kernel(double* R, const unsigned long long* __restrict__ L,
+                                                                  size_t lowest, const short* __restrict__ ex, int nkc,
+                                                                  int b) {
+  const int b2 = b * b, i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= nkc * b2) return;
+  const int w = i / b2, l = i - w * b2, l1 = l / b, l2 = l - l1 * b;
+  const size_t r0 = (size_t)blockIdx.y * nkc * b2;
+  const long long hi = reinterpret_cast<const long long*>(R)[r0 + i];
+  const long long lo = (long long)L[r0 + i], lw = (long long)L[lowest + r0 + i];
+  R[r0 + i] = ((double)hi + ((double)lo + (double)lw * 0x1p-54) * 0x1p-54) *
+              det_pow2(-ex[r0 + ((size_t)l2 * b + l1) * nkc + w]);
 }
 
 // ---------------------------------------------------------------------------
@@ -1485,7 +1498,8 @@ cudaError_t launch_delta_fused(const CombineArgs& a, cudaStream_t s, int mode) {
   if (!a.M1 || !a.M2 || (a.R1p && !a.M1p) || (a.R2p && !a.M2p)) return cudaErrorInvalidValue;
   if (mode == 1) return launch_delta_fused_mode<1>(a, s);
   if (mode == 2) return launch_delta_fused_mode<2>(a, s);
-  if (mode == 3 && a.det_scale && a.err) return launch_delta_fused_mode<3>(a, s);
+  if (mode == 3 && a.det_exp && a.det_lowest && a.err)
+    return a.R1p ? launch_delta_fused_mode<4>(a, s) : launch_delta_fused_mode<3>(a, s);
   return cudaErrorInvalidValue;
 }
 
@@ -1496,45 +1510,51 @@ cudaError_t launch_delta_finalize(double* R, const unsigned long long* M, size_t
   return cudaGetLastError();
 }
 
-size_t delta_scale_doubles(int nrows, int b, bool marginals) {
-  return (size_t)2 * (marginals ? 4 : 2) * nrows * b * b;  // scales, then bounds
+size_t delta_exp_count(const Geometry& geo, int nrows, bool marginals) {
+  return (size_t)(marginals ? 4 : 2) * nrows * geo.nkc * geo.b * geo.b;
 }
 
-cudaError_t launch_delta_scale(const CombineArgs& a, double* work, cudaStream_t s) {
-  const int b = a.geo.b, n = (a.R1p ? 4 : 2) * a.nrows * b * b;
-  unsigned long long* bnd = reinterpret_cast<unsigned long long*>(work + n);
-  cudaError_t e = cudaMemsetAsync(bnd, 0, (size_t)n * sizeof(double), s);
-  if (e != cudaSuccess) return e;
-  const dim3 grid(b * b, a.nrows);
-#define ALD_BOUND(BB)                                                                 \
-  if (a.v3sq_f32) delta_bound_kernel<BB><<<grid, 256, 0, s>>>(a, a.v3sq_f32, bnd);     \
-  else delta_bound_kernel<BB><<<grid, 256, 0, s>>>(a, a.v3sq, bnd);
+cudaError_t launch_delta_exp(const CombineArgs& a, cudaStream_t s) {
+  const int b = a.geo.b;
+  if (!a.brange || !a.occt || !a.err || !a.det_exp) return cudaErrorInvalidValue;
+  // R's in two launches, half the bands l2 each: callers tell the one-pass form
+  // from the two-pass one by the number of launches
+  const int h = b / 2;
+  const dim3 all((a.geo.nkc + 255) / 256, b, a.nrows), g0(all.x, h, a.nrows), g1(all.x, b - h, a.nrows);
+#define ALD_BOUND(BB, V)                                        \
+  delta_bound_kernel<BB, false><<<g0, 256, 0, s>>>(a, V, 0);    \
+  delta_bound_kernel<BB, false><<<g1, 256, 0, s>>>(a, V, h);    \
+  if (a.R1p) delta_bound_kernel<BB, true><<<all, 256, 0, s>>>(a, V, 0);
+#define ALD_BOUNDS(BB)         \
+  if (a.v3sq_f32) {            \
+    ALD_BOUND(BB, a.v3sq_f32)  \
+  } else {                     \
+    ALD_BOUND(BB, a.v3sq)      \
+  }
   if (b <= 3) {
-    ALD_BOUND(3)
+    ALD_BOUNDS(3)
   } else if (b <= 6) {
-    ALD_BOUND(6)
+    ALD_BOUNDS(6)
   } else if (b <= 12) {
-    ALD_BOUND(12)
+    ALD_BOUNDS(12)
   } else if (b <= kMaxBandsTet) {
-    ALD_BOUND(16)
+    ALD_BOUNDS(16)
   } else {
     return cudaErrorInvalidValue;
   }
+#undef ALD_BOUNDS
 #undef ALD_BOUND
-  delta_scale_kernel<<<(n + 255) / 256, 256, 0, s>>>(a, bnd, work, n);
   return cudaGetLastError();
 }
 
 cudaError_t launch_delta_finalize_wide(const CombineArgs& a, cudaStream_t s) {
   const int b = a.geo.b, nkc = a.geo.nkc;
-  const size_t n = (size_t)a.nrows * nkc * b * b, nr = (size_t)a.nrows * b * b;
-  const int blocks = (int)std::min<size_t>((n + 255) / 256, 148 * 16);
-  delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R1, a.M1, a.det_scale, n, nkc, b);
-  delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R2, a.M2, a.det_scale + nr, n, nkc, b);
-  if (a.R1p) {
-    delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R1p, a.M1p, a.det_scale + 2 * nr, n, nkc, b);
-    delta_finalize_wide_kernel<<<blocks, 256, 0, s>>>(a.R2p, a.M2p, a.det_scale + 3 * nr, n, nkc, b);
-  }
+  const size_t n = (size_t)a.nrows * nkc * b * b;
+  const dim3 grid((unsigned)(((size_t)nkc * b * b + 255) / 256), a.nrows);
+  double* R[4] = {a.R1, a.R2, a.R1p, a.R2p};
+  const unsigned long long* M[4] = {a.M1, a.M2, a.M1p, a.M2p};
+  for (int k = 0; k < (a.R1p ? 4 : 2); ++k)
+    delta_finalize_wide_kernel<<<grid, 256, 0, s>>>(R[k], M[k], a.det_lowest, a.det_exp + k * n, nkc, b);
   return cudaGetLastError();
 }
 
