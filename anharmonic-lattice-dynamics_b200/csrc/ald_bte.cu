@@ -925,6 +925,7 @@ static int cg_rows_t(int n, int row0, int nrows, size_t ld, const T* dA, const d
     msg = "cg: allocation failed";
     return ALD_ERR_NOMEM;
   }
+  w.n = -1;  // partial and pnum have other sizes here: graphs captured with them are not to run again
   const int vec = ((uintptr_t)dA & 15u) == 0 && (ld * sizeof(T)) % 16 == 0;
   CgDev* st = reinterpret_cast<CgDev*>(w.st.p);
   auto product = [&](const double* v, const CgDev* stp) -> int {  // aux = A v, all rows
