@@ -160,14 +160,14 @@ std::string build_fc2(const System& S, Fc2Csr& F);
 // kept per device (after a device synchronisation, so no queued work still
 // uses them) and handed out again to an allocation of the same byte size:
 // contexts created one after another reuse their workspaces without
-// cudaMalloc/cudaFree.  The cache holds at most 32 GiB per device; when
-// cudaMalloc runs out of memory the device's cached blocks are released and
-// the allocation retried.  dev_trim releases every cached block.
+// cudaMalloc/cudaFree.  The cache holds at most 32 GiB per device: beyond, and
+// when cudaMalloc runs out of memory, the blocks that lay unused for longest go
+// back to the driver.  dev_trim releases every cached block.
 cudaError_t dev_alloc(void** p, size_t bytes);
 void dev_free(void* p, size_t bytes);
 void dev_trim();
 // Held while a stream of the library is being captured into a CUDA graph and
-// while dev_free synchronises the device, so that contexts driven from
+// while the cache synchronises the device or gives blocks back, so that contexts driven from
 // different host threads never synchronise the device during a capture.
 std::mutex& capture_mutex();
 

@@ -109,9 +109,10 @@ void ald_destroy(ald_ctx* ctx);
 /* Device blocks of any size freed by the library (ald_destroy, workspace
  * resizes) stay reserved in a per-device cache, up to 32 GiB per device, and
  * are reused by later allocations of the same size: a context created after
- * another one skips cudaMalloc.  The cache gives its blocks back when
- * cudaMalloc runs out of memory; ald_release_cached_memory returns all of them
- * to the driver now (no counterpart in the reference). */
+ * another one skips cudaMalloc.  At the limit, and when cudaMalloc runs out of
+ * memory, the blocks unused for longest go back to the driver;
+ * ald_release_cached_memory returns all of them now (no counterpart in the
+ * reference). */
 void ald_release_cached_memory(void);
 int ald_get_info(ald_ctx* ctx, ald_info* info);
 
