@@ -189,15 +189,14 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   const bool fused = !gauss && v3_layout != 2 && delta_fused_supported(c->geo);
   // deterministic option: the fused delta with fixed-point sums (the same bits
   // on every run); their low parts, or the two-pass form's largest terms, need
-  // a buffer of the chunk's R1/R2 (and R1p/R2p) size.  The one-pass form's rare
-  // second run is not for ranks that exchange: they keep to two passes
+  // a buffer of the chunk's R1/R2 (and R1p/R2p) size
   const bool det = fused && (c->opt.deterministic > 0 ||
                              (c->opt.deterministic == ALD_DET_AUTO && c->opt.precision == ALD_FP64));
   // from 9 bands up the mixed V3 kernels write FP32
   const bool v3_large_f32 = v3_layout == 2 || (mixed && v3_tile_used(c));
   // more than 16 bands, or FP32 |V3|^2: the band-generic delta kernels, straight into R1/R2
   const bool any = !fused && (b > kDeltaSmallBands || v3_large_f32);
-  const bool wide = det && !sh && !c->det_two_pass;
+  bool wide = det && !c->det_two_pass;
   // the mixed pipeline hands |V3|^2 to the delta in FP32 where the delta
   // reads it so: from 9 bands up, and the class-form V3 of 3 and 6 bands into
   // the fused tetrahedron delta.  Half the bytes, twice the rows per chunk.
@@ -226,8 +225,21 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
                        c->v3c_re == re && c->v3c_layout == v3_layout && c->v3c_f32 == v3f && c->v3c_ptr == v3.p &&
                        c->v3c_n == v3.n;
   c->v3c_epoch = 0;
-  for (int r0 = rb; r0 < re; r0 += K) {
-    int nr = std::min(K, re - r0);
+  // sh: whether the one-pass delta of these rows found a term beyond its scale
+  auto overflowed = [&](bool* yes) -> int {
+    int h = 0;
+    ALD_CK(cudaMemcpyAsync(&h, c->err.p, sizeof h, cudaMemcpyDeviceToHost, s));
+    ALD_CK(cudaStreamSynchronize(s));
+    *yes = (h & 64) != 0;
+    if (!*yes) return ALD_OK;
+    h &= ~64;  // the other flags stay for the end of the call, after the exchanges
+    ALD_CK(cudaMemcpyAsync(c->err.p, &h, sizeof h, cudaMemcpyHostToDevice, s));
+    ALD_CK(cudaStreamSynchronize(s));
+    return ALD_OK;
+  };
+  int nr = 0;
+  for (int r0 = rb; r0 < re; r0 += nr) {
+    nr = std::min(K, re - r0);
     ALD_CK(tm.begin(1));
     if (!v3_kept && !v3_gauss) {
       V3Args va = v3_args(c, r0, nr, v3.p);
@@ -325,6 +337,18 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
       res->launches[2] += gauss ? 1 : 3;
     }
     ALD_CK(tm.end());
+    if (sh && wide && r0 + nr == re) {
+      // a rank cannot run the whole call again, with its exchanges, when the
+      // others do not: its own rows once more, in two passes
+      bool again = false;
+      r = overflowed(&again);
+      if (r) return r;
+      if (again) {
+        wide = false;
+        r0 = rb;
+        nr = 0;
+      }
+    }
   }
   // ---- 3: Q, Q_N, Q_U from the band sums
   double* dQ = Q.p;
