@@ -489,11 +489,38 @@ static int v3_line_alloc(ald_ctx* c, int nrows) {
   return ALD_OK;
 }
 
-int v3_gauss_rows(ald_ctx* c) {
-  if (!v3_line_supported(c->geo, v3_line_tables(c), c->opt.precision)) return 0;
+// rows whose class sums and line sums fit one chunk's bytes.  Per |V3|^2 byte
+// the line sums go as 1/N2: a third at 16^3 rock-salt, several times it where
+// the last axis has few points
+static int v3_line_rows(const ald_ctx* c) {
   const size_t per_row = v3_hbuf_bytes(c->geo.b, c->VC.ncls, 1, ALD_FP64) +
                          v3_line_row_bytes(c->geo, v3_line_tables(c), c->opt.precision);
   return (int)std::max<size_t>(1, std::min<size_t>(chunk_budget(c) / per_row, (size_t)c->T.nibz));
+}
+
+int v3_gauss_rows(ald_ctx* c) {
+  return v3_line_supported(c->geo, v3_line_tables(c), c->opt.precision) ? v3_line_rows(c) : 0;
+}
+
+// |V3|^2 of a's rows from line sums, by launch(args), as many rows at a time as v3_line_rows
+template <class Launch>
+static int run_v3_lines(ald_ctx* c, const V3Args& a0, int per_batch, Launch launch, int* nl, cudaError_t* e) {
+  const int K = std::min(v3_line_rows(c), a0.nrows);
+  const int r = v3_line_alloc(c, K);
+  if (r) return r;
+  const size_t row = (size_t)c->T.nkc * c->geo.b * c->geo.b * c->geo.b;
+  *e = cudaSuccess;
+  for (int r0 = 0; r0 < a0.nrows && *e == cudaSuccess; r0 += K) {
+    V3Args a = a0;
+    a.hbuf = c->w_h.p;
+    a.n1_first = a0.n1_first + r0;
+    a.nrows = std::min(K, a0.nrows - r0);
+    if (a.v3sq_f32) a.v3sq_f32 = a0.v3sq_f32 + (size_t)r0 * row;
+    else a.v3sq = a0.v3sq + (size_t)r0 * row;
+    *e = launch(a);
+    *nl += per_batch;
+  }
+  return ALD_OK;
 }
 
 int run_v3_gauss(ald_ctx* c, const V3Args& a0, const CombineArgs& ca, int* nlaunch) {
@@ -563,18 +590,17 @@ int run_v3(ald_ctx* c, const V3Args& a0, int* nlaunch) {
     nl += 1 + 3 * (int)(((long long)a.nrows * c->geo.nkc + per - 1) / per);
   } else if (v3_line_supported(c->geo, v3_line_tables(c), prec)) {
     // 3 bands: class sums axis by axis
-    const int r = v3_line_alloc(c, a.nrows);
+    // (launches: mode factors, class sums H, plane sums, the line kernel)
+    const int r = run_v3_lines(c, a, 4, [&](const V3Args& x) {
+      return launch_v3_line(x, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
+    }, &nl, &e);
     if (r) return r;
-    a.hbuf = c->w_h.p;
-    e = launch_v3_line(a, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
-    nl += 4;  // mode factors, class sums H, plane sums, the line kernel
   } else if (v3_pair_lines_supported(c->geo, v3_line_tables(c))) {
     // 6 bands: class sums axis by axis, mode products per pair
-    const int r = v3_line_alloc(c, a.nrows);
+    const int r = run_v3_lines(c, a, 3, [&](const V3Args& x) {
+      return launch_v3_pair_lines(x, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
+    }, &nl, &e);
     if (r) return r;
-    a.hbuf = c->w_h.p;
-    e = launch_v3_pair_lines(a, v3_line_tables(c), c->w_v3work.p, prec, c->stream);
-    nl += 3;
   } else if (v3_pair_supported(c->geo.b, prec)) {
     const size_t need = v3_hbuf_bytes(c->geo.b, c->VC.ncls, a.nrows, prec);
     if (c->w_h.n < need) CKA(c->w_h.alloc(need));
