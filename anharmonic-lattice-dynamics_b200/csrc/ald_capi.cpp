@@ -523,6 +523,22 @@ static int run_v3_lines(ald_ctx* c, const V3Args& a0, int per_batch, Launch laun
   return ALD_OK;
 }
 
+size_t v3_workspace_bytes(const ald_ctx* c, int nrows) {
+  const int b = c->geo.b, ncls = c->VC.ncls, prec = c->opt.precision;
+  const size_t soft = prec == ALD_MIXED && b >= 9 ? (size_t)256 << 20 : 0;  // v3_soft_fp64's GEMMs
+  const size_t gemm = c->tune_gemm_bytes ? c->tune_gemm_bytes : (size_t)2 << 30;
+  if (v3_tile_used(c)) return v3_tile_work_bytes(c->geo, ncls, nrows, prec) + soft;
+  if (prec == ALD_MIXED && v3_dense_tc_supported(b))
+    return v3_hbuf_bytes(b, ncls, nrows, prec) + v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) + gemm + soft;
+  if (v3_dense_supported(b)) return v3_hbuf_bytes(b, ncls, nrows, ALD_FP64) + ((size_t)2 << 30);
+  const V3LineTables t = v3_line_tables(c);
+  if (v3_line_supported(c->geo, t, prec) || v3_pair_lines_supported(c->geo, t)) {
+    const int k = std::min(v3_line_rows(c), nrows);
+    return v3_hbuf_bytes(b, ncls, k, ALD_FP64) + v3_line_work_bytes(c->geo, t, k, prec);
+  }
+  return v3_hbuf_bytes(b, ncls, nrows, ALD_FP64);
+}
+
 int run_v3_gauss(ald_ctx* c, const V3Args& a0, const CombineArgs& ca, int* nlaunch) {
   const int r = v3_line_alloc(c, a0.nrows);
   if (r) return r;

@@ -116,6 +116,8 @@ int v3_layout(const ald_ctx* c);
 // the chunk's byte budget), 0 where the cell has no such kernel
 int v3_gauss_rows(ald_ctx* c);
 int run_v3_gauss(ald_ctx* c, const V3Args& a, const CombineArgs& ca, int* nlaunch);
+// what run_v3 allocates for nrows rows, |V3|^2 itself left out (an upper estimate)
+size_t v3_workspace_bytes(const ald_ctx* c, int nrows);
 // g of cal_giso on the device (the element table unless ald_set_isotope_g set it)
 int ensure_giso(ald_ctx* c);
 KappaArgs kappa_args(ald_ctx* c, double tempk);

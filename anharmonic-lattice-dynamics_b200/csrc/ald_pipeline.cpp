@@ -609,20 +609,26 @@ static void release_pipeline_workspaces(ald_ctx* c) {
 }
 
 // An upper estimate of the device bytes one pipeline call on c allocates
-// beyond the context's tables: R1/R2, |V3|^2 of one chunk, the collision
-// matrix, the fixed-point sums of the deterministic delta, and for large
-// cells the V3 GEMM workspace (2 GiB at most) and the Householder
-// eigensolver's slots.  The batched entry point admits structures by it.
-static size_t pipeline_bytes_estimate(const ald_ctx* c) {
+// beyond the context's tables: eigenpairs, R1/R2, |V3|^2 of one chunk and what
+// V3 needs beside it, the collision matrix, the integer sums and scales of the
+// deterministic delta, and for large cells the Householder eigensolver's slots.
+// The batched entry point admits structures by it.
+static size_t pipeline_bytes_estimate(ald_ctx* c) {
   const size_t nibz = c->T.nibz, nkc = c->T.nkc, b = c->geo.b;
-  const size_t rsz = nibz * nkc * b * b * sizeof(double);
-  const size_t per_row = nkc * b * b * b * sizeof(double);
-  const size_t budget = c->opt.chunk_bytes ? c->opt.chunk_bytes : (size_t)512 << 20;
-  const size_t k = std::max<size_t>(1, std::min<size_t>(budget / per_row, nibz));
+  const size_t rsz = nkc * b * b * sizeof(double);  // R1 of one row
+  const size_t per_row = rsz * b;
+  const bool mixed = c->opt.precision != ALD_FP64;
+  // the mixed chunk takes twice the rows where |V3|^2 is FP32
+  const size_t rows = rows_per_chunk(c), k = mixed ? std::min(nibz, 2 * rows) : rows;
   const size_t N = 3 * b * nibz;
-  size_t s = 2 * rsz + k * per_row + N * N * sizeof(double);
-  s += 2 * (k * nkc * b * b) * sizeof(unsigned long long);  // deterministic delta
-  if (b > 12) s += c->tune_gemm_bytes ? c->tune_gemm_bytes : (size_t)2 << 30;
+  size_t s = nkc * (2 * b * b + 20 * b) * sizeof(double);
+  s += 2 * nibz * rsz + rows * per_row + N * (N + 4) * sizeof(double) / (mixed ? 2 : 1);
+  s += v3_workspace_bytes(c, (int)k);
+  if (delta_mode(c) == ALD_DELTA_GAUSS) s += combine_scratch_bytes(c->geo, (int)k, 1);
+  else if (!delta_fused_supported(c->geo) && b <= (size_t)kDeltaSmallBands)
+    s += combine_scratch_bytes(c->geo, (int)k, 0);
+  else if (c->opt.deterministic > 0 || (c->opt.deterministic == ALD_DET_AUTO && !mixed))
+    s += 4 * k * rsz + delta_exp_count(c->geo, (int)k, false) * sizeof(short);
   if (b > 64) s += heev_work_doubles((int)b, heev_slots((int)nkc * 7)) * sizeof(double);
   return s + ((size_t)256 << 20);
 }

@@ -48,3 +48,26 @@ def test_rows_in_batches(ald_lib, workdir, atoms, mesh):
     for o in out[1:]:
         for k in ("Q", "QN", "QU"):
             assert np.array_equal(o[k], out[0][k]), k
+
+
+def test_batch_on_a_nearly_full_device(ald_lib, workdir):
+    """Six structures of about 3.1 GB each with 9 GB free: the batched entry point starts as many at once as fit."""
+    torch = pytest.importorskip("torch")
+    d = make_ortho(workdir, 2, (32, 32, 2), delta="tetra")
+    opts = ald_lib.default_options(precision=ald_lib.FP64)
+    ctxs = [ald_lib.Context(d, opts) for _ in range(6)]
+    gc.collect()
+    ald_lib.release_cached_memory()
+    torch.cuda.empty_cache()
+    ballast = torch.empty(torch.cuda.mem_get_info()[0] - (9 << 30), dtype=torch.uint8, device="cuda")
+    try:
+        out, status = ald_lib.kappa_batched(ctxs, [300.0] * 6)
+    finally:
+        del ballast
+        torch.cuda.empty_cache()
+        for c in ctxs:
+            c.close()
+        ald_lib.release_cached_memory()
+    assert status == [0] * 6
+    for o in out[1:]:
+        assert np.array_equal(o["kappa_rta"], out[0]["kappa_rta"], equal_nan=True)
