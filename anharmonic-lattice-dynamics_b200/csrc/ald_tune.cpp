@@ -10,8 +10,8 @@
 // the current choice:
 //   1. the |V3|^2 chunk (IBZ rows per V3 and delta launch; 256 MiB .. 2 GiB,
 //      within a quarter of the free device memory);
-//   2. mixed path, 9 bands and up: the pair-batch workspace of the
-//      tensor-core mode-product GEMMs (launch count against L2 reuse).
+//   2. mixed cells whose V3 the tensor-core mode-product GEMMs form: their
+//      pair-batch workspace (launch count against L2 reuse).
 // The best choice stays on the context and goes into the cache file as one
 // line "<shape> chunk_bytes=.. rpc=.. wg=.. gemm_bytes=.. ms=..", replaced
 // in place when the shape is tuned again; a later call for the same shape
@@ -220,7 +220,7 @@ int ald_autotune(ald_ctx* c, const char* cache_path, double budget_s, ald_tuning
     if (r) break;
   }
   // 2. large cells: the GEMM pair-batch workspace
-  if (!r && c->opt.precision == ALD_MIXED && v3_dense_tc_supported(c->geo.b)) {
+  if (!r && c->opt.precision == ALD_MIXED && v3_dense_tc_supported(c->geo.b) && !v3_tile_used(c)) {
     const Choice base = best;
     for (size_t mb : {512, 1024, 4096}) {
       Choice ch = base;

@@ -307,8 +307,8 @@ int ald_kappa_batched(int n, ald_ctx* const* ctx, const double* tempk, ald_kappa
  * pipeline's autotuner.  ald_autotune times whole ald_kappa_pipeline calls
  * (device time, at the tmin of latdyn.params) over candidate launch shapes,
  * one knob at a time: the |V3|^2 chunk (IBZ rows per V3 and delta launch),
- * and for mixed cells of 9 bands and up the pair-batch workspace of
- * the tensor-core mode-product GEMMs.  It keeps the fastest on the context
+ * and for mixed cells whose V3 the tensor-core mode-product GEMMs form
+ * their pair-batch workspace.  It keeps the fastest on the context
  * and in the cache file (cache_path; NULL or "": $ALD_TUNE_CACHE; neither:
  * no file), one text line per shape (device, bands, mesh, IBZ rows,
  * precision, delta, deterministic option).  When the file already holds the
