@@ -461,7 +461,8 @@ static int v3_soft_fp64(ald_ctx* c, const V3Args& a, int* nl) {
 }
 
 // device bytes of one chunk of IBZ rows
-static size_t chunk_budget(const ald_ctx* c) { return c->opt.chunk_bytes ? c->opt.chunk_bytes : (size_t)512 << 20; }
+constexpr size_t kChunkBytes = (size_t)512 << 20;
+static size_t chunk_budget(const ald_ctx* c) { return c->opt.chunk_bytes ? c->opt.chunk_bytes : kChunkBytes; }
 
 static V3LineTables v3_line_tables(const ald_ctx* c) {
   V3LineTables t;
@@ -500,6 +501,17 @@ static int v3_line_rows(const ald_ctx* c) {
 
 int v3_gauss_rows(ald_ctx* c) {
   return v3_line_supported(c->geo, v3_line_tables(c), c->opt.precision) ? v3_line_rows(c) : 0;
+}
+
+// |V3|^2 rows within a byte budget
+static size_t rows_of(const ald_ctx* c, size_t budget) {
+  const size_t per_row = (size_t)c->T.nkc * c->geo.b * c->geo.b * c->geo.b * sizeof(double);
+  return std::max<size_t>(1, std::min<size_t>(budget / per_row, (size_t)c->T.nibz));
+}
+
+bool v3_gauss_used(ald_ctx* c) {
+  return delta_mode(c) == ALD_DELTA_GAUSS && v3_gauss_rows(c) > 0 &&
+         (size_t)c->T.nibz > rows_of(c, c->chunk_asked ? c->chunk_asked : kChunkBytes);
 }
 
 // |V3|^2 of a's rows from line sums, by launch(args), as many rows at a time as v3_line_rows
@@ -680,10 +692,7 @@ int delta_mode(ald_ctx* c) { return c->opt.delta; }
 double gauss_width(ald_ctx* c) { return c->opt.width_cm > 0 ? c->opt.width_cm : c->S.width; }
 
 // |V3|^2 rows per chunk within the byte budget
-int rows_per_chunk(ald_ctx* c) {
-  size_t per_row = (size_t)c->T.nkc * c->geo.b * c->geo.b * c->geo.b * sizeof(double);
-  return (int)std::max<size_t>(1, std::min<size_t>(chunk_budget(c) / per_row, (size_t)c->T.nibz));
-}
+int rows_per_chunk(ald_ctx* c) { return (int)rows_of(c, chunk_budget(c)); }
 
 }  // namespace capi
 }  // namespace ald
@@ -738,6 +747,7 @@ int ald_create_from_dir(const char* dir, const ald_options* opt, ald_ctx** out) 
   int ndev = 0;
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return fail(ALD_ERR_CUDA, "no CUDA device");
   c->device = c->opt.device;
+  c->chunk_asked = c->opt.chunk_bytes;
   CK(cudaSetDevice(c->device));
   CK(cudaStreamCreateWithFlags(&c->own_stream, cudaStreamNonBlocking));
   c->stream = c->own_stream;

@@ -82,6 +82,7 @@ struct ald_ctx {
   DevBuf<short> w_dexp;     // deterministic delta: the exponent of each R entry's scale
   bool det_overflow = false;  // a term was beyond the one-pass form's scale (check_err_flags)
   bool det_two_pass = false;  // take the two-pass form
+  size_t chunk_asked = 0;  // opt.chunk_bytes as the context was created with, whatever the tuner set since
   // launch shapes chosen by ald_autotune (0 = the built-in choices)
   int tune_v3_rpc = 0, tune_v3_wg = 0;  // kept for ald_set_tuning's callers; nothing reads them
   size_t tune_gemm_bytes = 0;
@@ -115,6 +116,10 @@ int v3_layout(const ald_ctx* c);
 // V3 and the Gaussian delta in one pass: rows per chunk (their line sums within
 // the chunk's byte budget), 0 where the cell has no such kernel
 int v3_gauss_rows(ald_ctx* c);
+// whether the pipeline takes it: where |V3|^2 of all rows does not fit one
+// chunk.  By the bytes that the context was created with, so that neither the
+// tuner's chunk nor a rank's share of the rows changes the arithmetic
+bool v3_gauss_used(ald_ctx* c);
 int run_v3_gauss(ald_ctx* c, const V3Args& a, const CombineArgs& ca, int* nlaunch);
 // what run_v3 allocates for nrows rows, |V3|^2 itself left out (an upper estimate)
 size_t v3_workspace_bytes(const ald_ctx* c, int nrows);

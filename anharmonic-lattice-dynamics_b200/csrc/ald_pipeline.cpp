@@ -207,8 +207,8 @@ static int run_pipeline_once(ald_ctx* c, double tempk, ald_kappa_result* res, do
   // cell with a kernel for V3 and the Gaussian delta together never stores it
   // (its chunks are cut by that kernel's own workspace).  argon 32^3 mixed, V3
   // and delta: 19.4 ms in two kernels, 11.9 in one; 26^3 FP64: 14.8 and 8.5
-  const bool one_chunk = re - rb <= K;
-  const bool v3_gauss = gauss && !it && !one_chunk && v3_gauss_rows(c) > 0;
+  const bool v3_gauss = !it && v3_gauss_used(c);
+  const bool one_chunk = !v3_gauss && re - rb <= K;
   if (v3_gauss) K = v3_gauss_rows(c);
   if (!v3_gauss) ALD_CKA(v3.alloc(v3f ? (v3n + 1) / 2 : v3n));
   const size_t rchunk = (size_t)K * nkc * b * b;  // entries of one chunk's R1
