@@ -903,13 +903,14 @@ __device__ __forceinline__ void delta_fused_body(const CombineArgs& a, const VT*
 
 // the kernels: the mixed one with the compiler's own register choice (55-62
 // registers at 6 bands, measured fastest), the FP64 one held to 64 registers
-// (8 CTAs per SM; measured fastest for it)
+// (8 CTAs per SM; measured fastest for it), with the marginals' scales to 80 (6
+// CTAs: 2.31 ms against 2.43 at 12^3 rock-salt)
 template <int B, class VT, int MODE>
 __global__ void __launch_bounds__(kFusedThreads) delta_fused_mixed_kernel(CombineArgs a, const VT* __restrict__ v3sq) {
   delta_fused_body<B, true, VT, MODE>(a, v3sq);
 }
 template <int B, int MODE>
-__global__ void __launch_bounds__(kFusedThreads, 8) delta_fused_fp64_kernel(CombineArgs a,
+__global__ void __launch_bounds__(kFusedThreads, MODE == 4 ? 6 : 8) delta_fused_fp64_kernel(CombineArgs a,
                                                                             const double* __restrict__ v3sq) {
   delta_fused_body<B, false, double, MODE>(a, v3sq);
 }
