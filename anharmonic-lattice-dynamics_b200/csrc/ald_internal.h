@@ -351,7 +351,7 @@ cudaError_t launch_v3_pair_lines(const V3Args& a, const V3LineTables& t, void* w
 // [row][line][slot 3][be ga][l1] complex (3 bands: [l1][be ga])
 cudaError_t launch_v3_lines(const V3Args& a, const V3LineTables& t, void* lines, int precision, cudaStream_t s);
 bool v3_lines_supported(const Geometry& g, const V3LineTables& t);
-// row stage alone, H in FP32 or FP64
+// row stage alone, H in FP64
 cudaError_t launch_v3_rows_f64(const V3Args& a, cudaStream_t s);
 // more than 12 bands (ald_v3_dense.cu): the class sums and both mode products
 // as batched complex GEMMs per (q1, q2) pair; hbuf from launch_v3_rows_f64;
@@ -390,7 +390,7 @@ struct CombineArgs {
   const int* mapinv;
   const double* v3sq;        // v3_layout 0: [row][q2][l1][l2][l3]; 1: [row][l2][l3][l1][q2]
   int v3_layout;
-  const float* v3sq_f32 = nullptr;  // FP32 |V3|^2 in place of v3sq (band-generic kernels only)
+  const float* v3sq_f32 = nullptr;  // FP32 |V3|^2 in place of v3sq (fused and band-generic deltas)
   const double* freq;        // [q][l]
   const double* dist;        // [q][l]
   const double* occt = nullptr;  // freq, then dist, as [l][q] (delta_gauss_pair)

@@ -494,8 +494,8 @@ __global__ void __launch_bounds__(256) q_from_r_kernel(Geometry g, int n1_first,
 // sets bit 64 of the error flag, as a weight beyond kDetCap does (a tetrahedron
 // of energies within 1e-6 cm^-1 around omega1), and the pipeline takes MODE 1
 // and 2.
-// Rock-salt 16^3 FP64: 14.3 ms in two passes, 8.1 in one (B200; with the
-// queue's two ends, below).
+// Rock-salt 16^3 FP64: 14.3 ms in two passes, 7.4 in one (B200; with the
+// queue's two ends, below), 5.5 in MODE 0.
 // corners of make_kp_reg_tet's six tetrahedra (c = o0 + 2 o1 + 4 o2), 3 bits
 // each, tetrahedra 0..4 in one word; tetrahedron 5 is (2, 5, 6, 7)
 constexpr unsigned long long kTetCornerCode =

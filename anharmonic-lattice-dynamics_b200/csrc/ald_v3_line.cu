@@ -23,8 +23,9 @@
 // with one sum over the classes per pair (ald_v3_pair.cu), 4.8 here.  Mixed
 // 32^3, 1768 rows: 10.6 ms with the class sums as split-FP16 tcgen05 MMAs,
 // 8.0 here, and the linewidths' error against 64 bits falls from 8.5e-7 to
-// 3.2e-8.  The line kernel is bound by issue and latency (FP32: issue slots
-// 58 % busy, 96 to 128 registers; FP64: FP64 pipe 35 to 38 %).
+// 3.2e-8.  The line kernel is bound by issue and latency (with the Gaussian
+// delta, FP32: issue slots 62 % busy, 128 registers, 16 warps per SM; FP64:
+// FP64 pipe 34 %, 168 registers, 12 warps).
 //
 // Steps 1 and 2 are in FP64 in both precisions; ALD_MIXED rounds H3 to FP32
 // and runs step 3 and the mode products in FP32, as the pair kernel runs its
@@ -112,9 +113,8 @@ __global__ void v3_line_modes_kernel(const double* __restrict__ w2, const double
     for (int k = i; k < 3 * n; k += gridDim.x * blockDim.x) e[k] = make_float2((float)ev[k].x, (float)ev[k].y);
 }
 
-// Steps 1 and 2.  A CTA takes one row, one m_0 and a tile of cw of the 9 b
-// components (be ga, l1); H2 of the tile stays in shared memory while m_1
-// runs.  About a sixth of the line kernel's time (argon 26^3, 299 rows: 0.22
+// Steps 1 and 2.  A CTA takes one row and one m_0; H2 of all 9 b components
+// (be ga, l1) stays in shared memory while m_1 runs.  About a sixth of the line kernel's time (argon 26^3, 299 rows: 0.22
 // of 1.23 ms); bound by the phase and H2 loads.
 constexpr int kPlaneThreads = 256, kPlaneM = 4;
 template <class C, int COMPS>

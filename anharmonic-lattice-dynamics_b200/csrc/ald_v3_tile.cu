@@ -21,8 +21,8 @@
 // formed alone has the same bits as in a chunk.  Sums are reordered against
 // the reference: agreement to rounding.
 //
-// Bound by issue and latency (24 bands FP32: issue slots 50 % busy, FMA pipe
-// 36 %, 18 warps per SM; 12 bands FP64: FP64 pipe 32 %).  Of the FP32 work at
+// Bound by issue and latency (24 bands FP32: issue slots 56 % busy, FMA pipe
+// 39 %, 17 warps per SM; 12 bands FP64: FP64 pipe 37 %, 14 warps).  Of the FP32 work at
 // 24 bands the class sums are a sixth of the products.
 #include <cuda_runtime.h>
 

@@ -68,7 +68,7 @@ typedef struct ald_options {
   size_t chunk_bytes;/* device bytes for one chunk of |V3|^2 rows (0 = automatic)      */
   int deterministic; /* the pipeline's tetrahedron delta (up to 16 bands):
                         1: sums with the same bits on every run (fixed-point integer
-                        atomics; about 1.4x the delta's time),
+                        atomics; about 1.35x the delta's time, mixed 1.65x),
                         0: FP64 atomics in arrival order (last bits vary between runs),
                         ALD_DET_AUTO (-1, the default): 1 for ALD_FP64, 0 otherwise    */
 } ald_options;
